@@ -434,7 +434,8 @@ int plan_aggregate_order(int64_t n, const int32_t* hptr, const int32_t* hidx, co
 
 int build_two_level(int64_t n, const int32_t* indptr, const int32_t* indices, const double* k64,
                     const int32_t* seg_row, int nseg, int nvc, void* mem, size_t bytes,
-                    PcgPrecondDesc<float>* pc, cudaStream_t stream, const int32_t* lab_in, int agg_target) {
+                    PcgPrecondDesc<float>* pc, cudaStream_t stream, const int32_t* lab_in, int agg_target,
+                    std::vector<int32_t>* h_seg_agg, std::vector<int32_t>* h_agg_ptr) {
   nvc = std::max(nvc, 1);
   if (bytes < two_level_bytes(n, seg_row, nseg, nvc)) return LAPY_ERR_WORKSPACE;
   std::vector<int32_t> lab(n, -1), nc(nseg, 0);
@@ -649,6 +650,8 @@ int build_two_level(int64_t n, const int32_t* indptr, const int32_t* indices, co
   }
   // the host vectors are pageable: the copies complete before they go away
   LAPY_CUDA_TRY(cudaStreamSynchronize(stream));
+  if (h_seg_agg) *h_seg_agg = seg_agg;
+  if (h_agg_ptr) *h_agg_ptr = agg_ptr;
   pc->kind = kPrecTwoLevel;
   pc->nagg = nagg;
   pc->agg = d_agg;

@@ -1141,24 +1141,33 @@ static int eigs_run(const EigPlan& P, const EigPtrs& e, const int32_t* indptr, c
   K.tuning = P.pcg;
   K.n = n; K.nnz = P.nnz; K.indptr = indptr; K.indices = indices;
   K.k64 = e.k64; K.k32 = e.k32; K.dinv64 = e.dinv64; K.dinv32 = e.dinv32;
-  {
+  // inner solves: on chip when every mesh fits, else the persistent PCG on
+  // SELL copies of K
+  std::vector<int32_t> h_seg_agg, h_agg_ptr;
+  if (P.precond == kPrecTwoLevel)
+    LAPY_TRY(build_two_level(n, indptr, indices, e.k64, P.ct.h_seg_row.data(), ns, P.ct.nvc, e.tl_mem,
+                             e.tl_bytes, &K.pc32, st, reorder ? lab.data() : nullptr, P.agg_target, &h_seg_agg,
+                             &h_agg_ptr));
+  ClusterPlan cluster;
+  if (P.precond != kPrecTwoLevel || K.pc32.agg_contig)
+    LAPY_TRY(cluster_plan(n, P.nnz, indptr, indices, e.k32, ns, P.ct.h_seg_row.data(),
+                          P.precond == kPrecTwoLevel ? h_seg_agg.data() : nullptr, h_agg_ptr.data(), p, e.sell_mem,
+                          e.sell_bytes, &cluster, st));
+  if (cluster.ok) {
+    K.cluster = &cluster;
+  } else {
     bool fits = false;
     LAPY_TRY(build_sell<float>(n, indptr, indices, e.k32, P.ct, e.sell_mem, e.sell_bytes, &K.sell32, &fits, st));
     if (!fits) K.sell32 = SellMatrix<float>();
-  }
-  {
-    bool fits = false;
     LAPY_TRY(build_sell<double>(n, indptr, indices, e.k64, P.ct, e.sell64_mem, e.sell64_bytes, &K.sell64, &fits, st));
     if (!fits) K.sell64 = SellMatrix<double>();
-    if (!m_is_diag) {
-      LAPY_TRY(build_sell<double>(n, indptr, indices, m_vals, P.ct, e.sellm_mem, e.sell64_bytes, &ops.sellM, &fits,
-                                  st));
-      if (!fits) ops.sellM = SellMatrix<double>();
-    }
   }
-  if (P.precond == kPrecTwoLevel)
-    LAPY_TRY(build_two_level(n, indptr, indices, e.k64, P.ct.h_seg_row.data(), ns, P.ct.nvc, e.tl_mem,
-                             e.tl_bytes, &K.pc32, st, reorder ? lab.data() : nullptr, P.agg_target));
+  if (!m_is_diag) {
+    bool fits = false;
+    LAPY_TRY(build_sell<double>(n, indptr, indices, m_vals, P.ct, e.sellm_mem, e.sell64_bytes, &ops.sellM, &fits,
+                                st));
+    if (!fits) ops.sellM = SellMatrix<double>();
+  }
 
   LAPY_CUDA_TRY(cudaMemsetAsync(e.rcnt, 0, 16, st));
   std::vector<int32_t> hact(ns, 1), hnsize(ns, 0);

@@ -51,6 +51,69 @@ static int residual64(const SysMatrix& K, const ChunkTable& ct, int p, const dou
   return csr_spmm<double>(K.n, K.indptr, K.indices, K.k64, p, X, R, -1.0, 1.0, G, stream);
 }
 
+// The whole refined solve on chip (pcg_cluster.cu); rn2, st and ctl are
+// ir_solve's workspace.
+static int ir_solve_cluster(const SysMatrix& K, int nsp, int p, const double* B, double* X, double rtol,
+                            int maxiter, double inner_rtol, int max_rounds, double* rn2, int32_t* st, void* ctl,
+                            cudaStream_t stream, IrStats* stats, double* relres2_host, int32_t* state_host) {
+  PcgPrecondDesc<float> pc = K.pc32;
+  ClusterSolve c;
+  c.n = K.n;
+  c.indptr = K.indptr;
+  c.indices = K.indices;
+  c.k64 = K.k64;
+  c.dinv = K.dinv32;
+  c.pc = &pc;
+  c.B = B;
+  c.X = X;
+  c.rtol = rtol;
+  c.inner_rtol = inner_rtol;
+  c.max_rounds = max_rounds;
+  c.maxiter = maxiter;
+  c.state = st;
+  c.relres2 = rn2;
+  c.ctl = (unsigned long long*)(((uintptr_t)ctl + 255) & ~uintptr_t(255));
+  LAPY_CUDA_TRY(cudaMemsetAsync(c.ctl, 0, 64, stream));
+  // segments without rows have no cluster: they are reported as solved
+  LAPY_CUDA_TRY(cudaMemsetAsync(st, 0, sizeof(int32_t) * nsp, stream));
+  LAPY_CUDA_TRY(cudaMemsetAsync(rn2, 0, sizeof(double) * nsp, stream));
+  const bool prof = lapy_profile_enabled();
+  cudaEvent_t e0 = nullptr, e1 = nullptr;
+  if (prof) {
+    LAPY_CUDA_TRY(cudaEventCreate(&e0));
+    LAPY_CUDA_TRY(cudaEventCreate(&e1));
+    LAPY_CUDA_TRY(cudaEventRecord(e0, stream));
+  }
+  LAPY_TRY(cluster_solve(*K.cluster, c, stream));
+  if (prof) LAPY_CUDA_TRY(cudaEventRecord(e1, stream));
+  std::vector<int32_t> hst(nsp);
+  unsigned long long hctl[8];
+  LAPY_CUDA_TRY(cudaMemcpyAsync(hst.data(), st, sizeof(int32_t) * nsp, cudaMemcpyDeviceToHost, stream));
+  if (relres2_host)
+    LAPY_CUDA_TRY(cudaMemcpyAsync(relres2_host, rn2, sizeof(double) * nsp, cudaMemcpyDeviceToHost, stream));
+  LAPY_CUDA_TRY(cudaMemcpyAsync(hctl, c.ctl, sizeof(hctl), cudaMemcpyDeviceToHost, stream));
+  LAPY_CUDA_TRY(cudaStreamSynchronize(stream));
+  if (prof) {
+    float ms = 0.f;
+    cudaEventElapsedTime(&ms, e0, e1);
+    cudaEventDestroy(e0);
+    cudaEventDestroy(e1);
+    lapy_profile_add_pcg(ms, (long long)hctl[0], (long long)hctl[2], (long long)hctl[3], K.cluster->np,
+                         (int)sizeof(float), pc.kind, (double)hctl[4], true);
+  }
+  IrStats local;
+  local.rounds = (int)hctl[1];
+  local.pcg_iters = (int64_t)hctl[0];
+  int worst = LAPY_OK;
+  for (int i = 0; i < nsp; ++i) {
+    if (state_host) state_host[i] = hst[i];
+    if (hst[i] != LAPY_OK && worst == LAPY_OK) worst = hst[i];
+  }
+  local.status = worst;
+  if (stats) *stats = local;
+  return LAPY_OK;
+}
+
 int ir_solve(const SysMatrix& K, const ChunkTable& ct, int p, const double* B, double* X,
              double rtol, int maxiter, int mixed, double inner_rtol, int max_rounds, void* ws,
              size_t ws_bytes, cudaStream_t stream, IrStats* stats, double* relres2_host,
@@ -70,6 +133,11 @@ int ir_solve(const SysMatrix& K, const ChunkTable& ct, int p, const double* B, d
   void* pws = w;
   const size_t pws_bytes = ws_bytes - (size_t)(w - (char*)ws);
   const int G = spmm_pick_group(n, K.nnz);
+
+  if (mixed && K.cluster && K.cluster->ok && K.cluster->p == p && !K.reliable &&
+      (precond == kPrecJacobi || precond == kPrecTwoLevel))
+    return ir_solve_cluster(K, nsp, p, B, X, rtol, maxiter, inner_rtol, max_rounds, rn2, st, pws, stream, stats,
+                            relres2_host, state_host);
 
   std::vector<double> hb(nsp), hr(nsp);
   std::vector<int32_t> hst(nsp), hmask(nsp, 0), final_st(nsp, LAPY_OK);
@@ -405,15 +473,22 @@ static int pcg_solve_impl(int64_t n, const int32_t* indptr, const int32_t* indic
     pc.ic_lev_b_row = plan.lev_b_row;
     K.pc32 = pc;
   }
-  if (mixed) {
-    bool fits = false;
-    LAPY_TRY(build_sell<float>(n, indptr, indices, k32, ct, sell_mem, sell_bytes, &K.sell32, &fits, stream));
-    if (!fits) K.sell32 = SellMatrix<float>();
-  }
+  ClusterPlan cluster;
+  bool have_sell = false;
   int64_t total_iters = 0;
   for (int c0 = 0; c0 < ncol; c0 += 16) {
     const int w = std::min(16, ncol - c0);
     const int p = next_pow2_le16(w);
+    // the matrix copy: packed for the on-chip solve when every segment fits
+    // (it depends on p), else SELL for the persistent PCG
+    if (mixed && !factored && !ic0 && cluster.p != p && !have_sell)
+      LAPY_TRY(cluster_plan(n, nnz, indptr, indices, k32, nseg, seg_row, nullptr, nullptr, p, sell_mem, sell_bytes,
+                            &cluster, stream));
+    K.cluster = cluster.ok ? &cluster : nullptr;
+    if (mixed && !cluster.ok && !have_sell) {
+      LAPY_TRY(build_sell<float>(n, indptr, indices, k32, ct, sell_mem, sell_bytes, &K.sell32, &have_sell, stream));
+      if (!have_sell) K.sell32 = SellMatrix<float>();
+    }
     LAPY_TRY(pack_cols(n, b, ncol, c0, w, p, Bp, stream));
     std::vector<double> rr(nseg * p);
     std::vector<int32_t> st(nseg * p);

@@ -1,7 +1,7 @@
 // Linear solves K X = B on a batch of segments: FP64 PCG, or FP32 PCG inside
 // FP64 iterative refinement (residuals recomputed in FP64 each round).
 #pragma once
-#include "pcg.cuh"
+#include "pcg_cluster.cuh"
 
 namespace lapy {
 
@@ -23,6 +23,7 @@ struct SysMatrix {
   // iterates), so the restarted rounds are the default.
   bool reliable = false;
   PcgTuning tuning;            // launch knobs of the persistent PCG
+  const ClusterPlan* cluster = nullptr;  // on-chip solve of this matrix (null or !ok: persistent PCG)
 };
 
 struct IrStats {
