@@ -14,6 +14,7 @@
 // possible and to keep every warp of the CTA busy.
 #include <cfloat>
 #include <cmath>
+#include "cluster.cuh"
 #include "dense.cuh"
 #include "dfloat.cuh"
 
@@ -478,9 +479,470 @@ __global__ void __launch_bounds__(kEigThreads, 4) sym_eig_kernel(double* Aall, i
   for (int q = t; q < want; q += kEigThreads) theta[q] = (q < nw) ? th[q] : 0.0;
 }
 
-int sym_eig_top(int nmat, double* A, int lda, const int32_t* nsize, int want, double* theta,
+// ---- the same eigensolver, one thread-block cluster per matrix -----------------
+// The one-CTA kernel above keeps its matrix in global memory: a step of the
+// Householder reduction is several passes over L2 with one CTA's loads in
+// flight, and FP64 (two results per clock and SM) of all its eigenvalues runs
+// on one SM.  Here the rows (double-float) are dealt round-robin to the CTAs
+// of a cluster and stay in shared memory.  A step has two cluster barriers: the
+// warp that owns row k forms the reflector and stores it in every CTA; every
+// warp multiplies its rows with it and stores the results w in every CTA; every
+// warp then updates its rows (w + K v formed in registers on the way), the one
+// that owns row k + 1 first, so that the next reflector is formed while the
+// other warps still update.  Eigenvalues, their inverse iteration (factors in
+// shared memory) and the back-transformation (one warp per vector, held in
+// registers) are split over the CTAs, clusters of close eigenvalues together.
+constexpr int kSymWarps = 16;
+
+__device__ __forceinline__ float2 df_mul(float2 a, float2 b) {
+  float h = 0.f, l = 0.f;
+  df_fma(a, b, h, l);
+  const float s = __fadd_rn(h, l);
+  return make_float2(s, __fsub_rn(l, __fsub_rn(s, h)));
+}
+// Sum of (h, l) over the warp's lanes, in every lane.
+__device__ __forceinline__ float2 df_warp_sum(float h, float l) {
+  const float s = __fadd_rn(h, l);
+  l = __fsub_rn(l, __fsub_rn(s, h));
+  h = s;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float bh = __shfl_xor_sync(0xffffffffu, h, o), bl = __shfl_xor_sync(0xffffffffu, l, o);
+    df_add(h, l, bh, bl);
+  }
+  return make_float2(h, l);
+}
+
+struct SymLayout {  // shared memory, byte offsets (rows: also the inverse iteration's factors)
+  int o_v, o_w, o_mail, o_d, o_e, o_e2, o_tau, o_th, o_flag, o_rows;
+  int rows_bytes;
+};
+
+template <int NC>  // 32 NC >= n
+__global__ void __launch_bounds__(32 * kSymWarps, 1) sym_eig_cluster_kernel(double* Aall, int lda, const int32_t* nsize,
+                                                                            int want, double* theta_all, double* S_all,
+                                                                            double* work_all, size_t wstride,
+                                                                            const int32_t* active, SymLayout lay) {
+  extern __shared__ __align__(16) unsigned char smx[];
+  __shared__ double s_bound[3], s_taud[2];
+  __shared__ int s_range[2];
+  const unsigned rank = cl_rank(), cs = cl_size();
+  const int b = blockIdx.x / cs;
+  if (active && !active[b]) return;  // every CTA of the cluster
+  const int n = nsize[b];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  double* A = Aall + (int64_t)b * lda * lda;
+  float2* Av = reinterpret_cast<float2*>(A);  // reflector k: row k, double-float
+  double* W = work_all + (int64_t)b * wstride;
+  double* theta = theta_all + (int64_t)b * want;
+  double* S = S_all + (int64_t)b * lda * want;
+  const int nw = min(want, n);
+  float2* vb = reinterpret_cast<float2*>(smx + lay.o_v);      // two reflectors (alternating)
+  float2* wb = reinterpret_cast<float2*>(smx + lay.o_w);      // tau A v
+  float2* mail = reinterpret_cast<float2*>(smx + lay.o_mail); // every warp's part of w'v
+  double* d = reinterpret_cast<double*>(smx + lay.o_d);
+  double* e = reinterpret_cast<double*>(smx + lay.o_e);
+  double* e2 = reinterpret_cast<double*>(smx + lay.o_e2);
+  float2* tau = reinterpret_cast<float2*>(smx + lay.o_tau);
+  double* th = reinterpret_cast<double*>(smx + lay.o_th);
+  int* flag = reinterpret_cast<int*>(smx + lay.o_flag);       // want: first of a cluster of eigenvalues
+  float2* Ar = reinterpret_cast<float2*>(smx + lay.o_rows);   // local row li: row li cs + rank
+
+  const int nloc = (n + (int)cs - 1 - (int)rank) / (int)cs;
+  for (int li = warp; li < nloc; li += kSymWarps) {
+    const double* src = A + (int64_t)(li * (int)cs + (int)rank) * lda;
+    for (int j = lane; j < n; j += 32) Ar[li * n + j] = df_split(src[j]);
+  }
+  cl_sync(cs);  // every CTA has read A (its rows are overwritten by reflectors) and runs
+
+  // reflector of row k (its owner's warp): d, e, tau and v to global memory, v
+  // and tau to every CTA
+  auto reflector = [&](int k) {
+    const float2* Ak = Ar + (k / (int)cs) * n;
+    double s2 = 0.0, x[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const int j = lane + 32 * c;
+      x[c] = (j > k && j < n) ? df_to_double(Ak[j]) : 0.0;
+      if (j > k + 1) s2 += x[c] * x[c];
+    }
+    s2 = warp_sum(s2);
+    const double alpha = df_to_double(Ak[k + 1]);
+    double beta = alpha, tk = 0.0, inv = 0.0;
+    if (s2 != 0.0) {
+      beta = -copysign(sqrt(alpha * alpha + s2), alpha);
+      tk = (beta - alpha) / beta;
+      inv = 1.0 / (alpha - beta);
+    }
+    if (lane == 0) {
+      W[k] = df_to_double(Ak[k]);
+      W[lda + k] = beta;
+      W[2 * lda + k] = tk;
+    }
+    float2* vk = vb + (k & 1) * n;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const int j = lane + 32 * c;
+      if (j > k && j < n) {
+        const float2 v = j == k + 1 ? make_float2(1.f, 0.f) : df_split(x[c] * inv);
+        Av[(int64_t)k * lda + j] = v;
+        for (unsigned r = 0; r < cs; ++r)
+          if (r == rank) vk[j] = v;
+          else cl_store2(cl_map(smem_u32(vk + j), r), v.x, v.y);
+      }
+    }
+    if (lane < (int)cs) {
+      if (lane == (int)rank) s_taud[k & 1] = tk;
+      else cl_store(cl_map(smem_u32(&s_taud[k & 1]), lane), tk);
+    }
+  };
+
+  // ---- 1. Householder tridiagonalisation
+  if (rank == 0 && warp == 0 && n > 2) reflector(0);
+  for (int k = 0; k + 2 < n; ++k) {
+    cl_sync(cs);
+    const int m0 = k + 1, c0 = m0 >> 5;
+    const float2* vk = vb + (k & 1) * n;
+    const float2 tk = df_split(s_taud[k & 1]);
+    float2 v[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const int j = lane + 32 * c;
+      v[c] = (j >= m0 && j < n) ? vk[j] : make_float2(0.f, 0.f);
+    }
+    // this warp's rows at or after m0 (local index = warp mod kSymWarps)
+    int l0 = m0 > (int)rank ? (m0 - (int)rank + (int)cs - 1) / (int)cs : 0;
+    l0 += (warp - l0) & (kSymWarps - 1);
+    // w = tau A v (two rows in flight) and w'v
+    float ph = 0.f, pl = 0.f;
+    for (int li = l0; li < nloc; li += 2 * kSymWarps) {
+      const bool two = li + kSymWarps < nloc;
+      const float2* A1 = Ar + li * n;
+      const float2* A2 = two ? A1 + kSymWarps * n : A1;
+      float h1 = 0.f, l1 = 0.f, h2 = 0.f, l2 = 0.f;
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        if (c >= c0) {
+          const int j = min(lane + 32 * c, n - 1);
+          df_fma(A1[j], v[c], h1, l1);
+          df_fma(A2[j], v[c], h2, l2);
+        }
+      }
+      const float2 w1 = df_mul(tk, df_warp_sum(h1, l1)), w2 = df_mul(tk, df_warp_sum(h2, l2));
+      const int i1 = li * (int)cs + (int)rank, i2 = i1 + kSymWarps * (int)cs;
+      df_fma(w1, vk[i1], ph, pl);
+      if (two) df_fma(w2, vk[i2], ph, pl);
+      if (lane < (int)cs) {
+        if (lane == (int)rank) {
+          wb[i1] = w1;
+          if (two) wb[i2] = w2;
+        } else {
+          cl_store2(cl_map(smem_u32(wb + i1), lane), w1.x, w1.y);
+          if (two) cl_store2(cl_map(smem_u32(wb + i2), lane), w2.x, w2.y);
+        }
+      }
+    }
+    if (lane < (int)cs) {
+      float2* at = mail + rank * kSymWarps + warp;
+      if (lane == (int)rank) *at = make_float2(ph, pl);
+      else cl_store2(cl_map(smem_u32(at), lane), ph, pl);
+    }
+    cl_sync(cs);
+    float kh = 0.f, kl = 0.f;
+    for (int i = lane; i < kSymWarps * (int)cs; i += 32) df_add(kh, kl, mail[i].x, mail[i].y);
+    const float2 K = df_mul(make_float2(-0.5f * tk.x, -0.5f * tk.y), df_warp_sum(kh, kl));
+    float2 w[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const int j = lane + 32 * c;
+      w[c] = (j >= m0 && j < n) ? wb[j] : make_float2(0.f, 0.f);
+      df_fma(K, v[c], w[c].x, w[c].y);
+    }
+    // A22 -= v w' + w v'
+    for (int li = l0; li < nloc; li += kSymWarps) {
+      const int i = li * (int)cs + (int)rank;
+      float2* Ai = Ar + li * n;
+      const float2 vi = vk[i];
+      float2 wi = wb[i];
+      df_fma(K, vi, wi.x, wi.y);
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        const int j = lane + 32 * c;
+        if (c >= c0 && j < n) {
+          float uh = 0.f, ul = 0.f;
+          df_fma(v[c], wi, uh, ul);
+          df_fma(w[c], vi, uh, ul);
+          float2 a = Ai[j];
+          df_add(a.x, a.y, -uh, -ul);
+          Ai[j] = a;
+        }
+      }
+      __syncwarp();
+      if (i == m0 && m0 + 2 < n) reflector(m0);
+    }
+  }
+  if (lane == 0) {  // the last two rows
+    for (int i = max(0, n - 2); i < n; ++i) {
+      if (i % (int)cs != (int)rank || (i / (int)cs) % kSymWarps != warp) continue;
+      const float2* Ai = Ar + (i / (int)cs) * n;
+      W[i] = df_to_double(Ai[i]);
+      W[lda + i] = i + 1 < n ? df_to_double(Ai[i + 1]) : 0.0;
+      W[2 * lda + i] = 0.0;
+    }
+  }
+  cl_sync(cs);
+  for (int i = t; i < n; i += blockDim.x) {
+    const double x = __ldcg(W + lda + i);
+    d[i] = __ldcg(W + i);
+    e[i] = x;
+    e2[i] = x * x;
+    tau[i] = df_split(__ldcg(W + 2 * lda + i));
+  }
+  __syncthreads();
+
+  // ---- 2. multisection for the nw largest eigenvalues, split over the CTAs
+  if (warp == 0) {
+    double lo = DBL_MAX, hi = -DBL_MAX, em = 0.0;
+    for (int i = lane; i < n; i += 32) {
+      const double r = (i > 0 ? fabs(e[i - 1]) : 0.0) + (i < n - 1 ? fabs(e[i]) : 0.0);
+      lo = fmin(lo, d[i] - r);
+      hi = fmax(hi, d[i] + r);
+      if (i < n - 1) em = fmax(em, e2[i]);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+      hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+      em = fmax(em, __shfl_xor_sync(0xffffffffu, em, o));
+    }
+    if (lane == 0) {
+      s_bound[0] = lo;
+      s_bound[1] = hi;
+      s_bound[2] = em;
+    }
+  }
+  __syncthreads();
+  double gl = s_bound[0], gu = s_bound[1];
+  const double tnorm = fmax(fabs(gl), fabs(gu));
+  const double pivmin = DBL_MIN * fmax(1.0, s_bound[2]) * 4.0;
+  gl -= 4.0 * DBL_EPSILON * tnorm + 2 * pivmin;
+  gu += 4.0 * DBL_EPSILON * tnorm + 2 * pivmin;
+  const int j0 = nw * (int)rank / (int)cs, j1 = nw * ((int)rank + 1) / (int)cs;
+  {
+    // lanes per eigenvalue: up to four warps in all (one per scheduler; more
+    // would queue for the FP64 pipe)
+    int G = 1;
+    while (G < 32 && 2 * G * (j1 - j0) <= 128) G *= 2;
+    const int ngroup = (int)blockDim.x / G, sub = t % G, gl0 = lane - sub;
+    const unsigned gmask = (G == 32) ? 0xffffffffu : (((1u << G) - 1u) << gl0);
+    const double frac = 1.0 / (double)(G + 1);
+    for (int j = j0 + t / G; j < j1; j += ngroup) {
+      const int idx = n - 1 - j;  // index from the bottom
+      double lo = gl, hi = gu;
+      for (int itb = 0; itb < 200; ++itb) {
+        const double wd = hi - lo;
+        if (wd <= 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi)) + pivmin) break;
+        const double x = lo + (double)(sub + 1) * (wd * frac);
+        const bool le = sturm_count(d, e2, n, x) <= idx;
+        const unsigned m = (__ballot_sync(gmask, le) & gmask) >> gl0;
+        const int kk = (m == 0u) ? 0 : 32 - __clz(m);  // probes at or below the eigenvalue
+        const double nlo = (kk == 0) ? lo : lo + (double)kk * (wd * frac);
+        const double nhi = (kk == G) ? hi : lo + (double)(kk + 1) * (wd * frac);
+        if (nlo == lo && nhi == hi) break;
+        lo = nlo;
+        hi = nhi;
+      }
+      if (sub == 0) {
+        const double v = 0.5 * (lo + hi);
+        for (unsigned r = 0; r < cs; ++r)
+          if (r == rank) th[j] = v;
+          else cl_store(cl_map(smem_u32(th + j), r), v);
+      }
+    }
+  }
+  __syncwarp();
+  cl_sync(cs);
+
+  // ---- 3. inverse iteration; a cluster of close eigenvalues belongs to the CTA
+  // whose share holds its first member
+  const double ctol = 1e-7 * fmax(tnorm, DBL_MIN);
+  const double tiny = DBL_EPSILON * fmax(tnorm, DBL_MIN);
+  for (int j = t; j < nw; j += blockDim.x) flag[j] = (j == 0) || (th[j - 1] - th[j] > ctol);
+  __syncthreads();
+  if (t < 2) {
+    int j = t == 0 ? j0 : j1;
+    while (j < nw && !flag[j]) ++j;
+    s_range[t] = j;
+  }
+  __syncthreads();
+  const int qa = s_range[0], qb = s_range[1], cnt = qb - qa;
+  const bool on_chip = (int64_t)6 * (cnt | 1) * n * 8 <= lay.rows_bytes;
+  const int ldq = on_chip ? cnt | 1 : want;
+  double* vecw = W + 4 * lda + 2 * want;
+  double* fac = on_chip ? reinterpret_cast<double*>(Ar) : vecw + qa;
+  const int64_t fs = on_chip ? (int64_t)ldq * n : (int64_t)lda * want;
+  double *U0i = fac, *U1 = fac + fs, *U2 = fac + 2 * fs, *Lm = fac + 3 * fs, *Pv = fac + 4 * fs;
+  double* Y = on_chip ? fac + 5 * fs : S + qa;
+  for (int ql = t; ql < cnt; ql += blockDim.x) {
+    const int q = qa + ql;
+    int j = q;
+    while (j > 0 && !flag[j]) --j;
+    // members of a cluster get shifts a few ulps apart (as LAPACK dstein)
+    const double shift = th[q] - (double)(q - j) * 10.0 * DBL_EPSILON * fmax(fabs(th[j]), tnorm);
+    tri_factor(d, e, n, shift, U0i + ql, U1 + ql, U2 + ql, Lm + ql, Pv + ql, ldq, tiny);
+    for (int i = 0; i < n; ++i) {  // deterministic start vector
+      unsigned h = (unsigned)(i * 2654435761u) ^ (unsigned)(q * 40503u + 0x9e3779b9u);
+      h ^= h >> 15; h *= 2246822519u; h ^= h >> 13;
+      Y[(int64_t)i * ldq + ql] = ((double)(h & 0xffffff) / 16777216.0) - 0.5;
+    }
+  }
+  __syncthreads();
+  for (int itr = 0; itr < 4; ++itr) {
+    for (int ql = t; ql < cnt; ql += blockDim.x)
+      tri_solve(U0i + ql, U1 + ql, U2 + ql, Lm + ql, Pv + ql, n, ldq, Y + ql);
+    __syncthreads();
+    int c = 0;  // number of the cluster, dealt round-robin to the warps
+    for (int a0 = qa; a0 < qb; ++c) {
+      int a1 = a0 + 1;
+      while (a1 < qb && !flag[a1]) ++a1;
+      if (c % kSymWarps == warp) {
+        for (int m = a0 - qa; m < a1 - qa; ++m) {
+          for (int r = a0 - qa; r < m; ++r) {
+            double dp = 0.0;
+            for (int i = lane; i < n; i += 32) dp += Y[(int64_t)i * ldq + r] * Y[(int64_t)i * ldq + m];
+            dp = warp_sum(dp);
+            for (int i = lane; i < n; i += 32) Y[(int64_t)i * ldq + m] -= dp * Y[(int64_t)i * ldq + r];
+          }
+          double nrm = 0.0;
+          for (int i = lane; i < n; i += 32) nrm += Y[(int64_t)i * ldq + m] * Y[(int64_t)i * ldq + m];
+          nrm = warp_sum(nrm);
+          const double inv = nrm > 0.0 ? 1.0 / sqrt(nrm) : 0.0;
+          for (int i = lane; i < n; i += 32) Y[(int64_t)i * ldq + m] *= inv;
+        }
+      }
+      a0 = a1;
+    }
+    __syncthreads();
+  }
+
+  // ---- 4. back-transformation Y <- H_0 ... H_{n-3} Y, a warp per vector in
+  // double-float registers, the next reflector's loads in flight
+  for (int ql = warp; ql < cnt; ql += kSymWarps) {
+    float2 y[NC], v[NC], vn[NC];
+    auto load = [&](int k, float2 (&x)[NC]) {
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        const int j = lane + 32 * c;
+        x[c] = (k >= 0 && j > k && j < n) ? __ldcg(Av + (int64_t)k * lda + j) : make_float2(0.f, 0.f);
+      }
+    };
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const int j = lane + 32 * c;
+      y[c] = j < n ? df_split(Y[(int64_t)j * ldq + ql]) : make_float2(0.f, 0.f);
+    }
+    load(n - 3, v);
+    for (int k = n - 3; k >= 0; --k) {
+      load(k - 1, vn);
+      float h = 0.f, l = 0.f;
+#pragma unroll
+      for (int c = 0; c < NC; ++c) df_fma(v[c], y[c], h, l);
+      const float2 s = df_mul(tau[k], df_warp_sum(h, l));
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        float uh = 0.f, ul = 0.f;
+        df_fma(s, v[c], uh, ul);
+        df_add(y[c].x, y[c].y, -uh, -ul);
+        v[c] = vn[c];
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const int j = lane + 32 * c;
+      if (j < n) S[(int64_t)j * want + qa + ql] = df_to_double(y[c]);
+    }
+  }
+  // rows beyond n and columns beyond nw (if want > n) are zero
+  for (int64_t i = (int64_t)rank * blockDim.x + t; i < (int64_t)lda * want; i += (int64_t)cs * blockDim.x)
+    if (i / want >= n || i % want >= nw) S[i] = 0.0;
+  if (rank == 0)
+    for (int q = t; q < want; q += blockDim.x) theta[q] = (q < nw) ? th[q] : 0.0;
+}
+
+// Shared memory of the cluster kernel for matrices of up to n rows.
+static size_t sym_layout(int n, int cs, int want, SymLayout* lay) {
+  size_t off = 0;
+  auto take = [&](size_t bytes) {
+    const size_t o = off;
+    off += (bytes + 15) & ~size_t(15);
+    return (int)o;
+  };
+  lay->o_v = take(16 * (size_t)n);
+  lay->o_w = take(8 * (size_t)n);
+  lay->o_mail = take(8 * (size_t)kSymWarps * cs);
+  lay->o_d = take(8 * (size_t)n);
+  lay->o_e = take(8 * (size_t)n);
+  lay->o_e2 = take(8 * (size_t)n);
+  lay->o_tau = take(8 * (size_t)n);
+  lay->o_th = take(8 * (size_t)want);
+  lay->o_flag = take(4 * (size_t)want);
+  lay->rows_bytes = (int)(8 * (size_t)((n + cs - 1) / cs) * n);
+  lay->o_rows = take((size_t)lay->rows_bytes);
+  return off;
+}
+
+static int launch_sym_cluster(int nmat, int cs, int n, double* A, int lda, const int32_t* nsize, int want,
+                              double* theta, double* S, double* work, const int32_t* active, cudaStream_t stream,
+                              bool* launched) {
+  *launched = false;
+  constexpr size_t kMax = 226 * 1024;
+  SymLayout lay;
+  size_t smem = sym_layout(n, cs, want, &lay);
+  if (smem > kMax) return LAPY_OK;
+  // what is free goes to the inverse iteration's factors
+  lay.rows_bytes += (int)((kMax - smem) & ~size_t(15));
+  lay.rows_bytes = std::min<int64_t>(lay.rows_bytes, std::max<int64_t>(8 * (int64_t)((n + cs - 1) / cs) * n,
+                                                                      (int64_t)48 * ((want + cs - 1) / cs | 1) * n));
+  smem = (size_t)lay.o_rows + (size_t)lay.rows_bytes;
+  auto kern = n <= 128 ? sym_eig_cluster_kernel<4> : n <= 256 ? sym_eig_cluster_kernel<8> : sym_eig_cluster_kernel<12>;
+  LAPY_CUDA_TRY(cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMax));
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)(nmat * cs));
+  cfg.blockDim = dim3(32 * kSymWarps);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = (unsigned)cs;
+  attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  int resident = 0;
+  if (cudaOccupancyMaxActiveClusters(&resident, (const void*)kern, &cfg) != cudaSuccess || resident < 1) {
+    cudaGetLastError();
+    return LAPY_OK;
+  }
+  LAPY_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, A, lda, nsize, want, theta, S, work, sym_eig_work_doubles(lda, want),
+                                   active, lay));
+  *launched = true;
+  return lapy_check_launch("sym_eig_cluster_kernel");
+}
+
+int sym_eig_top(int nmat, double* A, int lda, const int32_t* nsize, int nmax, int want, double* theta,
                 double* S, double* work, const int32_t* active, cudaStream_t stream) {
   if (nmat <= 0) return LAPY_OK;
+  if (nmax > 0 && nmax <= 384 && nmax <= lda) {
+    // the smallest cluster whose CTAs hold the rows, doubled while CTAs keep
+    // 24 rows or more and all matrices still run at once
+    int cs = 1;
+    SymLayout lay;
+    while (cs < 8 && sym_layout(nmax, cs, want, &lay) > 226 * 1024) cs *= 2;
+    while (cs < 8 && nmat * cs * 2 <= 120 && nmax >= 48 * cs) cs *= 2;
+    bool launched = false;
+    LAPY_TRY(launch_sym_cluster(nmat, cs, nmax, A, lda, nsize, want, theta, S, work, active, stream, &launched));
+    if (launched) return LAPY_OK;
+  }
   // v and w of a reflector in FP64 and double-float (4 lda); partial dots,
   // scaled dots and the double-float reflector of the back-transformation
   // (6 want + lda)

@@ -29,6 +29,7 @@
 #include <algorithm>
 #include <cmath>
 #include <vector>
+#include "cluster.cuh"
 #include "pcg_cluster.cuh"
 #include "scan.cuh"
 
@@ -75,48 +76,6 @@ struct ClArgs {
   int o_z, o_p, o_rc, o_yc, o_up, o_wp, o_mail, o_tab, o_push, o_val, o_code, o_coarse;
   int zrows, prows;
 };
-
-// ---- cluster primitives ------------------------------------------------------
-__device__ __forceinline__ unsigned cl_rank() {
-  unsigned r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ unsigned cl_size() {
-  unsigned r;
-  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
-  return r;
-}
-// Barrier over the cluster's threads; releases and acquires shared memory of
-// all CTAs and global memory.
-__device__ __forceinline__ void cl_sync(unsigned cs) {
-  if (cs == 1) {
-    __syncthreads();
-  } else {
-    __syncwarp();
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-  }
-}
-__device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ unsigned cl_map(unsigned addr, unsigned rank) {
-  unsigned r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ void cl_store(unsigned addr, float v) {
-  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
-}
-__device__ __forceinline__ void cl_store2(unsigned addr, float a, float b) {
-  asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(a), "f"(b) : "memory");
-}
-__device__ __forceinline__ void cl_store(unsigned addr, double v) {
-  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
-}
-__device__ __forceinline__ void cl_store4(unsigned addr, float a, float b, float c, float d) {
-  asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d)
-               : "memory");
-}
 
 // Row `slot` of a z / p array of this CTA.
 // NP = 8 keeps two planes of four columns, so that 16-byte reads of
