@@ -513,8 +513,111 @@ __device__ __forceinline__ float2 df_warp_sum(float h, float l) {
   return make_float2(h, l);
 }
 
+// Sturm counts on the tridiagonal scaled to norm 1 (d, e2 = e^2 as pairs): in
+// FP32 from the leading parts, and in double-float (x = xh + xl).  Both count
+// the eigenvalues below x of a matrix within their rounding of this one; the
+// minors are rescaled as in sturm_count.
+__device__ __forceinline__ int sturm_count_f32(const float2* d, const float2* e2, int n, float x) {
+  float a = 1.f, b = d[0].x - x;
+  if (b == 0.f) b = -0x1p-60f;
+  int cnt = b < 0.f;
+  for (int i = 1; i < n; ++i) {
+    float c = fmaf(d[i].x - x, b, -e2[i - 1].x * a);
+    a = b;
+    if (c == 0.f) {
+      a = copysignf(1.f, b);
+      c = -0x1p-60f * a;
+    }
+    cnt += (__float_as_int(c) ^ __float_as_int(a)) < 0;
+    b = c;
+    const int em = max((__float_as_int(a) >> 23) & 0xff, (__float_as_int(b) >> 23) & 0xff);
+    if (em > 127 + 40 || em < 127 - 40) {
+      const float s = __int_as_float((254 - em) << 23);
+      a *= s;
+      b *= s;
+    }
+  }
+  return cnt;
+}
+__device__ __forceinline__ int sturm_count_df(const float2* d, const float2* e2, int n, float xh, float xl) {
+  float2 a = make_float2(1.f, 0.f), b = d[0];
+  df_add(b.x, b.y, -xh, -xl);
+  if (b.x == 0.f) b = make_float2(-0x1p-80f, 0.f);
+  int cnt = b.x < 0.f;
+  for (int i = 1; i < n; ++i) {
+    float2 t = d[i];
+    df_add(t.x, t.y, -xh, -xl);
+    float h = 0.f, l = 0.f;
+    df_fma(t, b, h, l);
+    df_fma(make_float2(-e2[i - 1].x, -e2[i - 1].y), a, h, l);
+    const float s0 = __fadd_rn(h, l);
+    float2 c = make_float2(s0, __fsub_rn(l, __fsub_rn(s0, h)));
+    a = b;
+    if (c.x == 0.f) {
+      a = make_float2(copysignf(1.f, b.x), 0.f);
+      c = make_float2(-0x1p-80f * a.x, 0.f);
+    }
+    cnt += (__float_as_int(c.x) ^ __float_as_int(a.x)) < 0;
+    b = c;
+    const int em = max((__float_as_int(a.x) >> 23) & 0xff, (__float_as_int(b.x) >> 23) & 0xff);
+    if (em > 127 + 24 || em < 127 - 24) {
+      const float s = __int_as_float((254 - em) << 23);
+      a.x *= s; a.y *= s;
+      b.x *= s; b.y *= s;
+    }
+  }
+  return cnt;
+}
+
+// As tri_factor and tri_solve with the swap flags as bytes and without the
+// second superdiagonal of U, which is e[k + 1] after a swap and zero otherwise
+// (33 instead of 48 bytes per entry: the factors fit into shared memory).
+__device__ void tri_factor_compact(const double* d, const double* e, int n, double theta, double* U0i, double* U1,
+                                   double* L, unsigned char* P, int ld, double tiny) {
+  double x0 = d[0] - theta, x1 = (n > 1) ? e[0] : 0.0;
+  for (int k = 0; k < n - 1; ++k) {
+    const double y0 = e[k], y1 = d[k + 1] - theta, y2 = (k + 2 < n) ? e[k + 1] : 0.0;
+    const bool sw = fabs(x0) < fabs(y0);
+    double p0 = sw ? y0 : x0;
+    const double p1 = sw ? y1 : x1;
+    if (fabs(p0) < tiny) p0 = (p0 < 0 ? -tiny : tiny);
+    const double r = 1.0 / p0;
+    const double l = (sw ? x0 : y0) * r;
+    const int o = k * ld;
+    P[o] = sw;
+    L[o] = l;
+    U0i[o] = r;
+    U1[o] = p1;
+    x0 = (sw ? x1 : y1) - l * p1;
+    x1 = sw ? -l * y2 : y2;
+  }
+  if (fabs(x0) < tiny) x0 = (x0 < 0 ? -tiny : tiny);
+  U0i[(n - 1) * ld] = 1.0 / x0;
+}
+__device__ void tri_solve_compact(const double* e, const double* U0i, const double* U1, const double* L,
+                                  const unsigned char* P, int n, int ld, double* y) {
+  double yk = y[0];
+  for (int k = 0; k < n - 1; ++k) {
+    const int o = k * ld;
+    double yn = y[o + ld];
+    if (P[o]) { const double t = yk; yk = yn; yn = t; }
+    y[o] = yk;
+    yk = yn - L[o] * yk;
+  }
+  double z1 = yk * U0i[(n - 1) * ld], z2 = 0.0;  // z_{k+1}, z_{k+2}
+  y[(n - 1) * ld] = z1;
+  for (int k = n - 2; k >= 0; --k) {
+    const int o = k * ld;
+    const double u2 = P[o] ? e[k + 1] : 0.0;  // (z2 = 0 at k = n - 2)
+    const double z = (y[o] - U1[o] * z1 - u2 * z2) * U0i[o];
+    y[o] = z;
+    z2 = z1;
+    z1 = z;
+  }
+}
+
 struct SymLayout {  // shared memory, byte offsets (rows: also the inverse iteration's factors)
-  int o_v, o_w, o_mail, o_d, o_e, o_e2, o_tau, o_th, o_flag, o_rows;
+  int o_v, o_w, o_mail, o_d, o_e, o_e2, o_ds, o_es, o_tau, o_th, o_flag, o_rows;
   int rows_bytes;
 };
 
@@ -522,9 +625,10 @@ template <int NC>  // 32 NC >= n
 __global__ void __launch_bounds__(32 * kSymWarps, 1) sym_eig_cluster_kernel(double* Aall, int lda, const int32_t* nsize,
                                                                             int want, double* theta_all, double* S_all,
                                                                             double* work_all, size_t wstride,
-                                                                            const int32_t* active, SymLayout lay) {
+                                                                            const int32_t* active, int exact, SymLayout lay) {
   extern __shared__ __align__(16) unsigned char smx[];
-  __shared__ double s_bound[3], s_taud[2];
+  __shared__ double s_bound[3];
+  __shared__ float2 s_tau[2];
   __shared__ int s_range[2];
   const unsigned rank = cl_rank(), cs = cl_size();
   const int b = blockIdx.x / cs;
@@ -543,6 +647,8 @@ __global__ void __launch_bounds__(32 * kSymWarps, 1) sym_eig_cluster_kernel(doub
   double* d = reinterpret_cast<double*>(smx + lay.o_d);
   double* e = reinterpret_cast<double*>(smx + lay.o_e);
   double* e2 = reinterpret_cast<double*>(smx + lay.o_e2);
+  float2* ds = reinterpret_cast<float2*>(smx + lay.o_ds);    // d and e^2 scaled to norm 1, double-float
+  float2* es = reinterpret_cast<float2*>(smx + lay.o_es);
   float2* tau = reinterpret_cast<float2*>(smx + lay.o_tau);
   double* th = reinterpret_cast<double*>(smx + lay.o_th);
   int* flag = reinterpret_cast<int*>(smx + lay.o_flag);       // want: first of a cluster of eigenvalues
@@ -559,32 +665,74 @@ __global__ void __launch_bounds__(32 * kSymWarps, 1) sym_eig_cluster_kernel(doub
   // and tau to every CTA
   auto reflector = [&](int k) {
     const float2* Ak = Ar + (k / (int)cs) * n;
-    double s2 = 0.0, x[NC];
+    const int ck = (k + 1) >> 5;
+    // all in double-float (an FP64 square root and division here were most of
+    // a step's time), the column scaled by a power of two to entries of at
+    // most 2: squares of entries at rounding level would leave FP32's range
+    float2 x[NC];
+    float big = 0.f;
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
       const int j = lane + 32 * c;
-      x[c] = (j > k && j < n) ? df_to_double(Ak[j]) : 0.0;
-      if (j > k + 1) s2 += x[c] * x[c];
+      x[c] = (c >= ck && j > k && j < n) ? Ak[j] : make_float2(0.f, 0.f);
+      big = fmaxf(big, fabsf(x[c].x));
     }
-    s2 = warp_sum(s2);
-    const double alpha = df_to_double(Ak[k + 1]);
-    double beta = alpha, tk = 0.0, inv = 0.0;
-    if (s2 != 0.0) {
-      beta = -copysign(sqrt(alpha * alpha + s2), alpha);
-      tk = (beta - alpha) / beta;
-      inv = 1.0 / (alpha - beta);
+    big = warp_max(big);
+    const int ex = (__float_as_int(big) >> 23) & 0xff;  // 0: the column is zero (or far below rounding)
+    const bool scale = ex > 0 && ex < 253;
+    const float sc = __int_as_float((scale ? 254 - ex : 127) << 23);
+    float h = 0.f, l = 0.f;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      x[c].x *= sc;
+      x[c].y *= sc;
+      if (c >= ck && lane + 32 * c > k + 1) df_fma(x[c], x[c], h, l);
     }
+    const float2 sum = df_warp_sum(h, l);
+    const float2 alpha = make_float2(Ak[k + 1].x * sc, Ak[k + 1].y * sc);
+    float2 beta = alpha, tk = make_float2(0.f, 0.f), inv = make_float2(0.f, 0.f);
+    if (scale && sum.x > 0.f) {
+      // square root and reciprocals from their FP32 values by Newton steps on
+      // the double-float residual
+      float2 tt = sum;
+      df_fma(alpha, alpha, tt.x, tt.y);
+      const float y0 = rsqrtf(tt.x);
+      float2 root = make_float2(tt.x * y0, 0.f);
+#pragma unroll
+      for (int it = 0; it < 2; ++it) {
+        float2 res = tt;
+        df_fma(make_float2(-root.x, -root.y), root, res.x, res.y);
+        df_add(root.x, root.y, 0.5f * y0 * (res.x + res.y), 0.f);
+      }
+      auto recip = [](float2 x) {
+        const float q = 1.f / x.x;
+        float2 e1 = make_float2(1.f, 0.f);
+        df_fma(make_float2(-q, 0.f), x, e1.x, e1.y);
+        float2 r = make_float2(q, 0.f);
+        df_add(r.x, r.y, q * (e1.x + e1.y), 0.f);
+        return r;
+      };
+      const bool neg = alpha.x < 0.f;
+      const float2 aa = neg ? make_float2(-alpha.x, -alpha.y) : alpha;
+      float2 den = aa;
+      df_add(den.x, den.y, root.x, root.y);
+      inv = recip(den);
+      if (neg) inv = make_float2(-inv.x, -inv.y);
+      beta = neg ? root : make_float2(-root.x, -root.y);
+      tk = df_mul(den, recip(root));  // (beta - alpha) / beta
+    }
+    const float rs = __int_as_float((scale ? ex : 127) << 23);  // 1 / sc
     if (lane == 0) {
       W[k] = df_to_double(Ak[k]);
-      W[lda + k] = beta;
-      W[2 * lda + k] = tk;
+      W[lda + k] = df_to_double(make_float2(beta.x * rs, beta.y * rs));
+      reinterpret_cast<float2*>(W)[2 * lda + k] = tk;
     }
     float2* vk = vb + (k & 1) * n;
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
       const int j = lane + 32 * c;
       if (j > k && j < n) {
-        const float2 v = j == k + 1 ? make_float2(1.f, 0.f) : df_split(x[c] * inv);
+        const float2 v = j == k + 1 ? make_float2(1.f, 0.f) : df_mul(x[c], inv);
         Av[(int64_t)k * lda + j] = v;
         for (unsigned r = 0; r < cs; ++r)
           if (r == rank) vk[j] = v;
@@ -592,8 +740,8 @@ __global__ void __launch_bounds__(32 * kSymWarps, 1) sym_eig_cluster_kernel(doub
       }
     }
     if (lane < (int)cs) {
-      if (lane == (int)rank) s_taud[k & 1] = tk;
-      else cl_store(cl_map(smem_u32(&s_taud[k & 1]), lane), tk);
+      if (lane == (int)rank) s_tau[k & 1] = tk;
+      else cl_store2(cl_map(smem_u32(&s_tau[k & 1]), lane), tk.x, tk.y);
     }
   };
 
@@ -603,7 +751,7 @@ __global__ void __launch_bounds__(32 * kSymWarps, 1) sym_eig_cluster_kernel(doub
     cl_sync(cs);
     const int m0 = k + 1, c0 = m0 >> 5;
     const float2* vk = vb + (k & 1) * n;
-    const float2 tk = df_split(s_taud[k & 1]);
+    const float2 tk = s_tau[k & 1];
     float2 v[NC];
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
@@ -696,7 +844,7 @@ __global__ void __launch_bounds__(32 * kSymWarps, 1) sym_eig_cluster_kernel(doub
     d[i] = __ldcg(W + i);
     e[i] = x;
     e2[i] = x * x;
-    tau[i] = df_split(__ldcg(W + 2 * lda + i));
+    tau[i] = __ldcg(reinterpret_cast<const float2*>(W) + 2 * lda + i);
   }
   __syncthreads();
 
@@ -726,30 +874,80 @@ __global__ void __launch_bounds__(32 * kSymWarps, 1) sym_eig_cluster_kernel(doub
   const double pivmin = DBL_MIN * fmax(1.0, s_bound[2]) * 4.0;
   gl -= 4.0 * DBL_EPSILON * tnorm + 2 * pivmin;
   gu += 4.0 * DBL_EPSILON * tnorm + 2 * pivmin;
+  const double rn = tnorm > 0.0 ? 1.0 / tnorm : 0.0;
+  for (int i = t; i < n; i += blockDim.x) {
+    ds[i] = df_split(d[i] * rn);
+    es[i] = df_split(e2[i] * rn * rn);
+  }
+  __syncthreads();
   const int j0 = nw * (int)rank / (int)cs, j1 = nw * ((int)rank + 1) / (int)cs;
   {
-    // lanes per eigenvalue: up to four warps in all (one per scheduler; more
-    // would queue for the FP64 pipe)
-    int G = 1;
-    while (G < 32 && 2 * G * (j1 - j0) <= 128) G *= 2;
+    // A group of G lanes per eigenvalue probes G interior points a round: in
+    // FP32 down to 2^-20 of the norm, from there, widened by the FP32 counts'
+    // error (8 eps; twice that is taken), in double-float to 2^-42.  FP64
+    // counts, which cost 20 times as much a round (270 ns a row of T), finish
+    // only where the eigenvalues are a result (`exact`), from a verified bracket.
+    int G = 2;
+    while (G < 32 && 2 * G * (j1 - j0) <= 256) G *= 2;
     const int ngroup = (int)blockDim.x / G, sub = t % G, gl0 = lane - sub;
     const unsigned gmask = (G == 32) ? 0xffffffffu : (((1u << G) - 1u) << gl0);
-    const double frac = 1.0 / (double)(G + 1);
+    const float frac = 1.f / (float)(G + 1);
     for (int j = j0 + t / G; j < j1; j += ngroup) {
       const int idx = n - 1 - j;  // index from the bottom
-      double lo = gl, hi = gu;
-      for (int itb = 0; itb < 200; ++itb) {
-        const double wd = hi - lo;
-        if (wd <= 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi)) + pivmin) break;
-        const double x = lo + (double)(sub + 1) * (wd * frac);
-        const bool le = sturm_count(d, e2, n, x) <= idx;
+      // probes at or below the eigenvalue, from each lane's count
+      auto below = [&](bool le) {
         const unsigned m = (__ballot_sync(gmask, le) & gmask) >> gl0;
-        const int kk = (m == 0u) ? 0 : 32 - __clz(m);  // probes at or below the eigenvalue
-        const double nlo = (kk == 0) ? lo : lo + (double)kk * (wd * frac);
-        const double nhi = (kk == G) ? hi : lo + (double)(kk + 1) * (wd * frac);
-        if (nlo == lo && nhi == hi) break;
-        lo = nlo;
-        hi = nhi;
+        return (m == 0u) ? 0 : 32 - __clz(m);
+      };
+      float fl = -1.0001f, fw = 2.0002f;
+      while (fw > 0x1p-20f) {
+        const int kk = below(sturm_count_f32(ds, es, n, fl + (float)(sub + 1) * (fw * frac)) <= idx);
+        fl += (float)kk * (fw * frac);
+        fw *= frac;
+      }
+      fl -= 0x1p-19f;
+      fw += 0x1p-18f;
+      float2 l2 = make_float2(fl, 0.f);
+      // the bracket holds: no more than idx below its lower end, more below its upper
+      const bool at_lo = sub == 0 ? sturm_count_df(ds, es, n, fl, 0.f) <= idx
+                                  : sub == 1 ? sturm_count_df(ds, es, n, fl + fw, 0.f) > idx : true;
+      const bool good = (__ballot_sync(gmask, at_lo) & gmask) == gmask;
+      double lo = gl, hi = gu;
+      if (good) {
+        while (fw > 0x1p-42f) {
+          float2 x = l2;
+          df_add(x.x, x.y, (float)(sub + 1) * (fw * frac), 0.f);
+          const int kk = below(sturm_count_df(ds, es, n, x.x, x.y) <= idx);
+          df_add(l2.x, l2.y, (float)kk * (fw * frac), 0.f);
+          fw *= frac;
+        }
+        lo = df_to_double(l2) * tnorm;
+        hi = lo + (double)fw * tnorm;
+      }
+      if (exact || !good) {
+        if (good) {  // widened by the double-float counts' error, then checked
+          const double wide = 0x1p-41 * tnorm;
+          const bool ok = sub == 0 ? sturm_count(d, e2, n, lo - wide) <= idx
+                                   : sub == 1 ? sturm_count(d, e2, n, hi + wide) > idx : true;
+          if ((__ballot_sync(gmask, ok) & gmask) == gmask) {
+            lo -= wide;
+            hi += wide;
+          } else {
+            lo = gl;
+            hi = gu;
+          }
+        }
+        for (int itb = 0; itb < 200; ++itb) {
+          const double wd = hi - lo;
+          if (wd <= 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi)) + pivmin) break;
+          const double step = wd / (double)(G + 1);
+          const int kk = below(sturm_count(d, e2, n, lo + (double)(sub + 1) * step) <= idx);
+          const double nlo = (kk == 0) ? lo : lo + (double)kk * step;
+          const double nhi = (kk == G) ? hi : lo + (double)(kk + 1) * step;
+          if (nlo == lo && nhi == hi) break;
+          lo = nlo;
+          hi = nhi;
+        }
       }
       if (sub == 0) {
         const double v = 0.5 * (lo + hi);
@@ -775,20 +973,21 @@ __global__ void __launch_bounds__(32 * kSymWarps, 1) sym_eig_cluster_kernel(doub
   }
   __syncthreads();
   const int qa = s_range[0], qb = s_range[1], cnt = qb - qa;
-  const bool on_chip = (int64_t)6 * (cnt | 1) * n * 8 <= lay.rows_bytes;
+  const bool on_chip = (int64_t)33 * (cnt | 1) * n <= lay.rows_bytes;
   const int ldq = on_chip ? cnt | 1 : want;
   double* vecw = W + 4 * lda + 2 * want;
   double* fac = on_chip ? reinterpret_cast<double*>(Ar) : vecw + qa;
   const int64_t fs = on_chip ? (int64_t)ldq * n : (int64_t)lda * want;
-  double *U0i = fac, *U1 = fac + fs, *U2 = fac + 2 * fs, *Lm = fac + 3 * fs, *Pv = fac + 4 * fs;
-  double* Y = on_chip ? fac + 5 * fs : S + qa;
+  double *U0i = fac, *U1 = fac + fs, *Lm = fac + 2 * fs;
+  double* Y = on_chip ? fac + 3 * fs : S + qa;
+  unsigned char* Pv = reinterpret_cast<unsigned char*>(on_chip ? fac + 4 * fs : vecw + 3 * fs) + (on_chip ? 0 : qa);
   for (int ql = t; ql < cnt; ql += blockDim.x) {
     const int q = qa + ql;
     int j = q;
     while (j > 0 && !flag[j]) --j;
     // members of a cluster get shifts a few ulps apart (as LAPACK dstein)
     const double shift = th[q] - (double)(q - j) * 10.0 * DBL_EPSILON * fmax(fabs(th[j]), tnorm);
-    tri_factor(d, e, n, shift, U0i + ql, U1 + ql, U2 + ql, Lm + ql, Pv + ql, ldq, tiny);
+    tri_factor_compact(d, e, n, shift, U0i + ql, U1 + ql, Lm + ql, Pv + ql, ldq, tiny);
     for (int i = 0; i < n; ++i) {  // deterministic start vector
       unsigned h = (unsigned)(i * 2654435761u) ^ (unsigned)(q * 40503u + 0x9e3779b9u);
       h ^= h >> 15; h *= 2246822519u; h ^= h >> 13;
@@ -798,7 +997,7 @@ __global__ void __launch_bounds__(32 * kSymWarps, 1) sym_eig_cluster_kernel(doub
   __syncthreads();
   for (int itr = 0; itr < 4; ++itr) {
     for (int ql = t; ql < cnt; ql += blockDim.x)
-      tri_solve(U0i + ql, U1 + ql, U2 + ql, Lm + ql, Pv + ql, n, ldq, Y + ql);
+      tri_solve_compact(e, U0i + ql, U1 + ql, Lm + ql, Pv + ql, n, ldq, Y + ql);
     __syncthreads();
     int c = 0;  // number of the cluster, dealt round-robin to the warps
     for (int a0 = qa; a0 < qb; ++c) {
@@ -883,6 +1082,8 @@ static size_t sym_layout(int n, int cs, int want, SymLayout* lay) {
   lay->o_d = take(8 * (size_t)n);
   lay->o_e = take(8 * (size_t)n);
   lay->o_e2 = take(8 * (size_t)n);
+  lay->o_ds = take(8 * (size_t)n);
+  lay->o_es = take(8 * (size_t)n);
   lay->o_tau = take(8 * (size_t)n);
   lay->o_th = take(8 * (size_t)want);
   lay->o_flag = take(4 * (size_t)want);
@@ -892,7 +1093,7 @@ static size_t sym_layout(int n, int cs, int want, SymLayout* lay) {
 }
 
 static int launch_sym_cluster(int nmat, int cs, int n, double* A, int lda, const int32_t* nsize, int want,
-                              double* theta, double* S, double* work, const int32_t* active, cudaStream_t stream,
+                              double* theta, double* S, double* work, const int32_t* active, bool exact, cudaStream_t stream,
                               bool* launched) {
   *launched = false;
   constexpr size_t kMax = 226 * 1024;
@@ -902,7 +1103,7 @@ static int launch_sym_cluster(int nmat, int cs, int n, double* A, int lda, const
   // what is free goes to the inverse iteration's factors
   lay.rows_bytes += (int)((kMax - smem) & ~size_t(15));
   lay.rows_bytes = std::min<int64_t>(lay.rows_bytes, std::max<int64_t>(8 * (int64_t)((n + cs - 1) / cs) * n,
-                                                                      (int64_t)48 * ((want + cs - 1) / cs | 1) * n));
+                                                                      (int64_t)33 * ((want + cs - 1) / cs | 1) * n));
   smem = (size_t)lay.o_rows + (size_t)lay.rows_bytes;
   auto kern = n <= 128 ? sym_eig_cluster_kernel<4> : n <= 256 ? sym_eig_cluster_kernel<8> : sym_eig_cluster_kernel<12>;
   LAPY_CUDA_TRY(cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMax));
@@ -924,13 +1125,13 @@ static int launch_sym_cluster(int nmat, int cs, int n, double* A, int lda, const
     return LAPY_OK;
   }
   LAPY_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, A, lda, nsize, want, theta, S, work, sym_eig_work_doubles(lda, want),
-                                   active, lay));
+                                   active, exact ? 1 : 0, lay));
   *launched = true;
   return lapy_check_launch("sym_eig_cluster_kernel");
 }
 
 int sym_eig_top(int nmat, double* A, int lda, const int32_t* nsize, int nmax, int want, double* theta,
-                double* S, double* work, const int32_t* active, cudaStream_t stream) {
+                double* S, double* work, const int32_t* active, bool exact, cudaStream_t stream) {
   if (nmat <= 0) return LAPY_OK;
   if (nmax > 0 && nmax <= 384 && nmax <= lda) {
     // the smallest cluster whose CTAs hold the rows, doubled while CTAs keep
@@ -940,7 +1141,7 @@ int sym_eig_top(int nmat, double* A, int lda, const int32_t* nsize, int nmax, in
     while (cs < 8 && sym_layout(nmax, cs, want, &lay) > 226 * 1024) cs *= 2;
     while (cs < 8 && nmat * cs * 2 <= 120 && nmax >= 48 * cs) cs *= 2;
     bool launched = false;
-    LAPY_TRY(launch_sym_cluster(nmat, cs, nmax, A, lda, nsize, want, theta, S, work, active, stream, &launched));
+    LAPY_TRY(launch_sym_cluster(nmat, cs, nmax, A, lda, nsize, want, theta, S, work, active, exact, stream, &launched));
     if (launched) return LAPY_OK;
   }
   // v and w of a reflector in FP64 and double-float (4 lda); partial dots,

@@ -1252,7 +1252,7 @@ static int eigs_run(const EigPlan& P, const EigPtrs& e, const int32_t* indptr, c
       LAPY_CUDA_TRY(cudaMemcpyAsync(e.nsize, hnsize.data(), 4 * ns, cudaMemcpyHostToDevice, st));
       copy_T_kernel<<<ns, 256, 0, st>>>(e.T, e.Tc, lda, m, e.active);
       LAPY_TRY(lapy_check_launch("copy_T_kernel"));
-      LAPY_TRY(sym_eig_top(ns, e.Tc, lda, e.nsize, m, keff, e.theta, e.S, e.eigw, e.active, st));
+      LAPY_TRY(sym_eig_top(ns, e.Tc, lda, e.nsize, m, keff, e.theta, e.S, e.eigw, e.active, false, st));
       conv_check_kernel<<<ns, 128, 0, st>>>(ns, p, m, lda, keff, k, tol, e.theta, e.S, e.Bm, e.fail, e.nconv,
                                             e.active, e.Sfinal, e.theta_final, e.resid);
       LAPY_TRY(lapy_check_launch("conv_check_kernel"));
@@ -1356,7 +1356,7 @@ static int eigs_run(const EigPlan& P, const EigPtrs& e, const int32_t* indptr, c
   LAPY_TRY(lapy_check_launch("rr_prepare_kernel"));
   std::vector<int32_t> hk(ns, keff);
   LAPY_CUDA_TRY(cudaMemcpyAsync(e.nsize, hk.data(), 4 * ns, cudaMemcpyHostToDevice, st));
-  LAPY_TRY(sym_eig_top(ns, e.Cneg, keff, e.nsize, keff, k, e.theta2, e.V, e.eigw2, nullptr, st));
+  LAPY_TRY(sym_eig_top(ns, e.Cneg, keff, e.nsize, keff, k, e.theta2, e.V, e.eigw2, nullptr, true, st));
   rr_finish_kernel<<<ns, 128, 0, st>>>(keff, k, e.Mk, e.V, e.theta2, evals);
   LAPY_TRY(lapy_check_launch("rr_finish_kernel"));
   // eigenvectors X V in double-float (X_df holds X; V split into S_df, which
