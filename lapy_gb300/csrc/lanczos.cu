@@ -82,17 +82,25 @@ __global__ void __launch_bounds__(256) gemm_tn_partial_kernel(BMat X, int na, BM
   if (a < na && b < nb) partial[((int64_t)c * na + a) * nb + b] = acc;
 }
 
-// out[s][a][b] (leading dim ldo) = sum over chunks of segment s
+// out[s][a][b] (leading dim ldo) = sum over chunks of segment s: eight lanes
+// per entry, lane k adding chunks k, k + 8, ... (four neighbouring entries per
+// warp read a chunk's partials together), then three exchanges.  One thread
+// per entry took 40 us for the 161 chunks of a 10,242-row mesh.
 __global__ void gemm_tn_reduce_kernel(const double* __restrict__ partial, int na, int nb,
                                       const int32_t* __restrict__ seg_chunk, double* __restrict__ out,
                                       int64_t out_seg_stride, int ldo) {
   const int s = blockIdx.x;
   const int c0 = seg_chunk[s], c1 = seg_chunk[s + 1];
-  for (int e = blockIdx.y * blockDim.x + threadIdx.x; e < na * nb; e += gridDim.y * blockDim.x) {
-    const int a = e / nb, b = e % nb;
+  const int lane = threadIdx.x & 31, k = lane >> 2;
+  const int64_t m = (int64_t)na * nb;
+  for (int64_t e0 = ((int64_t)blockIdx.y * blockDim.x + threadIdx.x) / 32 * 4; e0 < m;
+       e0 += (int64_t)gridDim.y * blockDim.x / 8) {
+    const int64_t e = e0 + (lane & 3);
     double acc = 0.0;
-    for (int c = c0; c < c1; ++c) acc += partial[((int64_t)c * na + a) * nb + b];
-    out[(int64_t)s * out_seg_stride + (int64_t)a * ldo + b] = acc;
+    if (e < m)
+      for (int c = c0 + k; c < c1; c += 8) acc += partial[(int64_t)c * m + e];
+    for (int o = 16; o >= 4; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (k == 0 && e < m) out[(int64_t)s * out_seg_stride + e / nb * ldo + e % nb] = acc;
   }
 }
 
@@ -121,58 +129,6 @@ __global__ void __launch_bounds__(256) gemm_nn_kernel(BMat X, int na, const doub
 // Block-row forms of the two basis products for a basis stored as blocks of P
 // columns (block j: n x P row-major at X + j * bst), one thread per row.
 //
-// TN: partial[c][j*P + a][b] = sum over chunk c's rows of X_j(row, a) Y(row, b)
-// for JB consecutive blocks per CTA (grid.y), accumulated in registers and
-// reduced over the CTA in a fixed order.
-template <int P, int JB>
-__global__ void __launch_bounds__(256) gemm_tn_blk_kernel(const double* __restrict__ X, int64_t bst, int nblk,
-                                                          const double* __restrict__ Y,
-                                                          const int32_t* __restrict__ chunk_row,
-                                                          const int32_t* __restrict__ chunk_seg,
-                                                          const int32_t* __restrict__ active,
-                                                          double* __restrict__ partial) {
-  constexpr int NV = JB * P * P;
-  __shared__ double red[8][NV];
-  const int c = blockIdx.x, j0 = blockIdx.y * JB;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  double acc[NV];
-#pragma unroll
-  for (int v = 0; v < NV; ++v) acc[v] = 0.0;
-  if (!active || active[chunk_seg[c]]) {
-    const int64_t r1 = chunk_row[c + 1];
-    for (int64_t r = chunk_row[c] + threadIdx.x; r < r1; r += blockDim.x) {
-      double y[P];
-#pragma unroll
-      for (int b = 0; b < P; ++b) y[b] = __ldg(Y + r * P + b);
-#pragma unroll
-      for (int jj = 0; jj < JB; ++jj) {
-        if (j0 + jj < nblk) {
-          const double* xr = X + (int64_t)(j0 + jj) * bst + r * P;
-#pragma unroll
-          for (int a = 0; a < P; ++a) {
-            const double x = __ldg(xr + a);
-#pragma unroll
-            for (int b = 0; b < P; ++b) acc[(jj * P + a) * P + b] = fma(x, y[b], acc[(jj * P + a) * P + b]);
-          }
-        }
-      }
-    }
-  }
-#pragma unroll
-  for (int v = 0; v < NV; ++v) {
-    const double t = warp_sum(acc[v]);
-    if (lane == 0) red[warp][v] = t;
-  }
-  __syncthreads();
-  const int na = nblk * P;
-  for (int v = threadIdx.x; v < NV; v += blockDim.x) {
-    double t = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w][v];
-    const int jj = v / (P * P), a = (v / P) % P, b = v % P;
-    if (j0 + jj < nblk) partial[((int64_t)c * na + (j0 + jj) * P + a) * P + b] = t;
-  }
-}
-
 // NN: Y(row, b) = beta Y(row, b) + alpha sum_j sum_a X_j(row, a) H_s[j*P + a][b]
 // with the segment's H (nblk*P x P) staged in shared memory.
 template <int P>
@@ -236,59 +192,170 @@ __global__ void to_df_inplace_kernel(int64_t m, double* x) {
   reinterpret_cast<float2*>(x)[i] = make_float2(h, __double2float_rn(v - (double)h));
 }
 
-// TN with the basis in double-float form (see gemm_tn_blk_kernel for the layout).
-template <int P, int JB>
+// Sums of NV double-float values over the warp's lanes l, l + TPR, l + 2 TPR,
+// ... (the 32 / TPR lanes of one residue mod TPR) by halving exchanges: NV - 1
+// exchanges or fewer instead of NV log2(32 / TPR).  Afterwards the lane holds
+// the sums of the values first .. first + left - 1 in its leading entries.
+template <int NV, int TPR>
+__device__ __forceinline__ int df_lane_totals(float (&h)[NV], float (&l)[NV], int& left) {
+  const int lane = threadIdx.x & 31;
+  int first = 0;
+  constexpr int LOG = (TPR == 1 ? 5 : TPR == 2 ? 4 : TPR == 4 ? 3 : 2);
+  left = NV;
+#pragma unroll
+  for (int st = 0; st < LOG; ++st) {
+    const int mask = 16 >> st;
+    const int half = NV >> (st + 1);
+    if (half > 0) {
+      const bool up = lane & mask;
+#pragma unroll
+      for (int i = 0; i < (NV >> (st + 1)); ++i) {
+        const float kh = up ? h[i + half] : h[i], kl = up ? l[i + half] : l[i];
+        const float sh = up ? h[i] : h[i + half], sl = up ? l[i] : l[i + half];
+        h[i] = kh;
+        l[i] = kl;
+        df_add(h[i], l[i], __shfl_xor_sync(0xffffffffu, sh, mask), __shfl_xor_sync(0xffffffffu, sl, mask));
+      }
+      first += up ? half : 0;
+      left = half;
+    } else {
+      df_add(h[0], l[0], __shfl_xor_sync(0xffffffffu, h[0], mask), __shfl_xor_sync(0xffffffffu, l[0], mask));
+    }
+  }
+  return first;
+}
+// The same in FP64.
+template <int NV, int TPR>
+__device__ __forceinline__ int f64_lane_totals(double (&v)[NV], int& left) {
+  const int lane = threadIdx.x & 31;
+  int first = 0;
+  constexpr int LOG = (TPR == 1 ? 5 : TPR == 2 ? 4 : TPR == 4 ? 3 : 2);
+  left = NV;
+#pragma unroll
+  for (int st = 0; st < LOG; ++st) {
+    const int mask = 16 >> st;
+    const int half = NV >> (st + 1);
+    if (half > 0) {
+      const bool up = lane & mask;
+#pragma unroll
+      for (int i = 0; i < (NV >> (st + 1)); ++i) {
+        const double keep = up ? v[i + half] : v[i], send = up ? v[i] : v[i + half];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, mask);
+      }
+      first += up ? half : 0;
+      left = half;
+    } else {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], mask);
+    }
+  }
+  return first;
+}
+
+// TN with the basis in double-float form: TPR lanes share a row, each taking
+// P / TPR of the block's columns (16 accumulators per lane at P = 8, so that
+// the sums over lanes cost 14 exchanges; one lane per row had 64 accumulators
+// and 320).  A warp's lanes read consecutive 16-byte pieces of X.  Bound by
+// the FP32 pipe (about 10 instructions per product) on large batches, by
+// latency on one mesh; per product 300 -> 11 us at 10,242 rows, 8 columns,
+// 128 basis vectors.
+template <int P, int TPR, int JB>
 __global__ void __launch_bounds__(256) gemm_tn_df_kernel(const float2* __restrict__ X, int64_t bst, int nblk,
                                                          const float2* __restrict__ Y,
                                                          const int32_t* __restrict__ chunk_row,
                                                          const int32_t* __restrict__ chunk_seg,
                                                          const int32_t* __restrict__ active,
                                                          double* __restrict__ partial) {
-  constexpr int NV = JB * P * P;
-  __shared__ double red[8][NV];
+  constexpr int PA = P / TPR;        // columns of X per lane
+  constexpr int NV = JB * PA * P;    // accumulators: [jj][a][b]
+  __shared__ double red[8][TPR][NV];
   const int c = blockIdx.x, j0 = blockIdx.y * JB;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int warp = threadIdx.x >> 5, sub = threadIdx.x % TPR;
   float sh[NV], sl[NV];
 #pragma unroll
   for (int v = 0; v < NV; ++v) { sh[v] = 0.f; sl[v] = 0.f; }
   if (!active || active[chunk_seg[c]]) {
     const int64_t r1 = chunk_row[c + 1];
-    for (int64_t r = chunk_row[c] + threadIdx.x; r < r1; r += blockDim.x) {
+    for (int64_t r = chunk_row[c] + threadIdx.x / TPR; r < r1; r += blockDim.x / TPR) {
       float2 y[P];
 #pragma unroll
       for (int b = 0; b < P; ++b) y[b] = __ldg(Y + r * P + b);
 #pragma unroll
       for (int jj = 0; jj < JB; ++jj) {
         if (j0 + jj < nblk) {
-          const float2* xr = X + (int64_t)(j0 + jj) * bst + r * P;
+          const float2* xr = X + (int64_t)(j0 + jj) * bst + r * P + sub * PA;
 #pragma unroll
-          for (int a = 0; a < P; ++a) {
+          for (int a = 0; a < PA; ++a) {
             const float2 x = xr[a];
 #pragma unroll
-            for (int b = 0; b < P; ++b) df_fma(x, y[b], sh[(jj * P + a) * P + b], sl[(jj * P + a) * P + b]);
+            for (int b = 0; b < P; ++b) df_fma(x, y[b], sh[(jj * PA + a) * P + b], sl[(jj * PA + a) * P + b]);
           }
         }
       }
     }
   }
 #pragma unroll
-  for (int v = 0; v < NV; ++v) {  // warp sum in double-float (FP32 instructions)
-    float h = __fadd_rn(sh[v], sl[v]);
-    float l = __fsub_rn(sl[v], __fsub_rn(h, sh[v]));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float bh = __shfl_xor_sync(0xffffffffu, h, o), bl = __shfl_xor_sync(0xffffffffu, l, o);
-      df_add(h, l, bh, bl);
-    }
-    if (lane == 0) red[warp][v] = (double)h + (double)l;
+  for (int v = 0; v < NV; ++v) {  // normalise before the two-sums
+    const float h = __fadd_rn(sh[v], sl[v]);
+    sl[v] = __fsub_rn(sl[v], __fsub_rn(h, sh[v]));
+    sh[v] = h;
   }
+  int left;
+  const int first = df_lane_totals<NV, TPR>(sh, sl, left);
+#pragma unroll
+  for (int i = 0; i < NV; ++i)
+    if (i < left) red[warp][sub][first + i] = (double)sh[i] + (double)sl[i];  // (equal sums from several lanes)
   __syncthreads();
   const int na = nblk * P;
-  for (int v = threadIdx.x; v < NV; v += blockDim.x) {
+  for (int e = threadIdx.x; e < TPR * NV; e += blockDim.x) {
+    const int s = e / NV, v = e % NV;
     double t = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w][v];
-    const int jj = v / (P * P), a = (v / P) % P, b = v % P;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) t += red[w][s][v];
+    const int jj = v / (PA * P), a = s * PA + (v / P) % PA, b = v % P;
     if (j0 + jj < nblk) partial[((int64_t)c * na + (j0 + jj) * P + a) * P + b] = t;
+  }
+}
+
+// P x P Gram matrices X' Y in FP64 (X, Y: n x P), split as gemm_tn_df_kernel.
+template <int P, int TPR>
+__global__ void __launch_bounds__(256) gram_f64_kernel(const double* __restrict__ X, const double* __restrict__ Y,
+                                                       const int32_t* __restrict__ chunk_row,
+                                                       const int32_t* __restrict__ chunk_seg,
+                                                       const int32_t* __restrict__ active,
+                                                       double* __restrict__ partial) {
+  constexpr int PA = P / TPR, NV = PA * P;
+  __shared__ double red[8][TPR][NV];
+  const int c = blockIdx.x;
+  const int warp = threadIdx.x >> 5, sub = threadIdx.x % TPR;
+  double acc[NV];
+#pragma unroll
+  for (int v = 0; v < NV; ++v) acc[v] = 0.0;
+  if (!active || active[chunk_seg[c]]) {
+    const int64_t r1 = chunk_row[c + 1];
+    for (int64_t r = chunk_row[c] + threadIdx.x / TPR; r < r1; r += blockDim.x / TPR) {
+      double y[P];
+#pragma unroll
+      for (int b = 0; b < P; ++b) y[b] = __ldg(Y + r * P + b);
+#pragma unroll
+      for (int a = 0; a < PA; ++a) {
+        const double x = __ldg(X + r * P + sub * PA + a);
+#pragma unroll
+        for (int b = 0; b < P; ++b) acc[a * P + b] = fma(x, y[b], acc[a * P + b]);
+      }
+    }
+  }
+  int left;
+  const int first = f64_lane_totals<NV, TPR>(acc, left);
+#pragma unroll
+  for (int i = 0; i < NV; ++i)
+    if (i < left) red[warp][sub][first + i] = acc[i];
+  __syncthreads();
+  for (int e = threadIdx.x; e < TPR * NV; e += blockDim.x) {
+    const int s = e / NV, v = e % NV;
+    double t = 0.0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) t += red[w][s][v];
+    partial[((int64_t)c * P + s * PA + v / P) * P + v % P] = t;
   }
 }
 
@@ -471,35 +538,47 @@ __global__ void reorth_mask_kernel(int nseg, int p, const double* __restrict__ n
   if (a && need) atomicAdd(&cnt[1], 1ull);
 }
 
-// Cholesky of the p x p Gram matrix of every segment: G = R' R (R upper).
-// Inactive segments get R = I.  fail[s] = 1 when G is not numerically SPD.
+// Cholesky of the p x p Gram matrix of every segment: G = R' R (R upper), one
+// warp per segment, lane i holding column i of R (p <= 16): a pivot's square
+// root and reciprocal are the chain, one of each per column (one thread did a
+// division per entry: 25 us at p = 8).  Inactive segments get R = I.
+// fail[s] = 1 when G is not numerically SPD.
 __global__ void chol_small_kernel(int nseg, int p, const double* __restrict__ G, double* __restrict__ R,
                                   const int32_t* __restrict__ active, int32_t* __restrict__ fail) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  const int s = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
+  const int lane = threadIdx.x & 31;
   if (s >= nseg) return;
   const double* g = G + (int64_t)s * p * p;
   double* r = R + (int64_t)s * p * p;
-  for (int i = 0; i < p * p; ++i) r[i] = 0.0;
   if (!active[s]) {
-    for (int i = 0; i < p; ++i) r[i * p + i] = 1.0;
+    for (int e = lane; e < p * p; e += 32) r[e] = (e / p == e % p) ? 1.0 : 0.0;
     return;
   }
-  double gmax = 0.0;
-  for (int i = 0; i < p; ++i) gmax = fmax(gmax, fabs(g[i * p + i]));
+  const int i = min(lane, p - 1);
+  double gmax = fabs(g[i * p + i]);
+  for (int o = 16; o > 0; o >>= 1) gmax = fmax(gmax, __shfl_xor_sync(0xffffffffu, gmax, o));
+  double col[16];  // rows j of column i, what is left of (G + G') / 2, then R
+#pragma unroll
+  for (int j = 0; j < 16; ++j) col[j] = j < p ? 0.5 * (g[j * p + i] + g[i * p + j]) : 0.0;
   int bad = 0;
-  for (int j = 0; j < p; ++j) {
-    double dsum = 0.5 * (g[j * p + j] + g[j * p + j]);
-    for (int k = 0; k < j; ++k) dsum -= r[k * p + j] * r[k * p + j];
-    if (!(dsum > 1e-28 * gmax) || !isfinite(dsum)) { bad = 1; dsum = fmax(gmax, 1e-300) * 1e-28; }
-    const double rjj = sqrt(dsum);
-    r[j * p + j] = rjj;
-    for (int i = j + 1; i < p; ++i) {
-      double v = 0.5 * (g[j * p + i] + g[i * p + j]);
-      for (int k = 0; k < j; ++k) v -= r[k * p + j] * r[k * p + i];
-      r[j * p + i] = v / rjj;
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    if (j < p) {
+      double d = __shfl_sync(0xffffffffu, col[j], j);
+      if (!(d > 1e-28 * gmax) || !isfinite(d)) { bad = 1; d = fmax(gmax, 1e-300) * 1e-28; }
+      const double rjj = sqrt(d), inv = 1.0 / rjj;
+      col[j] = i == j ? rjj : i > j ? col[j] * inv : 0.0;
+#pragma unroll
+      for (int k = j + 1; k < 16; ++k)
+        if (k < p) col[k] -= __shfl_sync(0xffffffffu, col[j], k) * col[j];
     }
   }
-  fail[s] = bad;
+  if (lane < p) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+      if (j < p) r[j * p + i] = col[j];
+  }
+  if (lane == 0) fail[s] = bad;
 }
 
 // W(row, :) = W(row, :) * R_s^-1  (R upper triangular, p x p): R and the
@@ -787,10 +866,11 @@ struct EigPlan {
   int64_t nagg_max = 0;
   ChunkTable ct;   // PCG chunks
   ChunkTable gt;   // GEMM chunks (larger)
+  ChunkTable tt;   // chunks of the Gram-Schmidt TN products (at least 512 rows where the mesh has them)
 };
 
 struct EigPtrs {
-  void* ct_mem; void* gt_mem;
+  void* ct_mem; void* gt_mem; void* tt_mem;
   int32_t* diag_pos; double* k64; float* k32; double* dinv64; float* dinv32;
   double* basis; float2* basis_df; double* Y; double* W; double* MW; float2* MW_df; float2* S_df; float2* X_df;
   void* ir_ws; size_t ir_bytes;
@@ -822,6 +902,10 @@ static void plan_eig(int64_t n, int64_t nnz, int nseg, const int32_t* seg_row, i
   // basis products: long chunks, so a CTA's register tiles sum many rows
   // before their one reduction
   plan_chunks(srow.data(), nseg, 2 * lapy_num_sms(), &P->gt, kGemmChunkRows);
+  // the TN products split over basis blocks too: a CTA sums at least 512 rows
+  // before its one reduction over the warp, which costs as much as eight rows
+  plan_chunks(srow.data(), nseg, (int)std::min<int64_t>(2 * lapy_num_sms(), std::max<int64_t>(1, n / 512)), &P->tt,
+              kGemmChunkRows);
 }
 
 static size_t layout_eig(const EigPlan& P, char* base, EigPtrs* q) {
@@ -836,6 +920,7 @@ static size_t layout_eig(const EigPlan& P, char* base, EigPtrs* q) {
   EigPtrs e;
   e.ct_mem = take(chunk_table_bytes(P.ct));
   e.gt_mem = take(chunk_table_bytes(P.gt));
+  e.tt_mem = take(chunk_table_bytes(P.tt));
   e.diag_pos = (int32_t*)take(4 * n);
   e.k64 = (double*)take(8 * nnz);
   e.k32 = (float*)take(4 * nnz);
@@ -856,7 +941,7 @@ static size_t layout_eig(const EigPlan& P, char* base, EigPtrs* q) {
   e.sell64_bytes = sell_bytes_bound(nnz, P.ct, sizeof(double));
   e.sell64_mem = take(e.sell64_bytes);
   e.sellm_mem = take(e.sell64_bytes);
-  const size_t part_elems = (size_t)P.gt.nchunk * std::max((size_t)lda * p, (size_t)keff * keff);
+  const size_t part_elems = (size_t)std::max(P.gt.nchunk, P.tt.nchunk) * std::max((size_t)lda * p, (size_t)keff * keff);
   e.partial = (double*)take(8 * part_elems);
   e.H = (double*)take(8 * (size_t)ns * lda * p);
   e.Hsum = (double*)take(8 * (size_t)ns * lda * p);
@@ -923,36 +1008,26 @@ struct EigOps {
       return LAPY_OK;
     return csr_spmm<double>(P.n, indptr, indices, m_vals, ncol, X, Y, 1.0, 0.0, G, st);
   }
-  // out_s (na x nb, ldo) = X' Y per segment
-  template <int PB, int JB>
-  int gemm_tn_blk(BMat X, int na, BMat Y, const int32_t* act) const {
-    const int nblk = na / PB;
-    dim3 grid(P.gt.nchunk, lapy_ceil_div(nblk, JB));
-    gemm_tn_blk_kernel<PB, JB><<<grid, 256, 0, st>>>(X.base, X.bst, nblk, Y.base, P.gt.chunk_row, P.gt.chunk_seg,
-                                                     act, e.partial);
-    return lapy_check_launch("gemm_tn_blk_kernel");
+  dim3 reduce_grid(int na, int nb) const {  // 32 entries per CTA of gemm_tn_reduce_kernel
+    return dim3(P.nseg, std::max(1u, std::min(256u, lapy_ceil_div((int64_t)na * nb, 32))));
   }
+  // out_s (na x nb, ldo) = X' Y per segment
   int gemm_tn(BMat X, int na, BMat Y, int nb, double* out, int64_t out_stride, int ldo, const int32_t* act) const {
-    const bool blk = X.bs == nb && Y.bs == nb && Y.bst == 0 && na % nb == 0;
-    if (blk && nb == 1) {
-      LAPY_TRY((gemm_tn_blk<1, 16>(X, na, Y, act)));
-    } else if (blk && nb == 2) {
-      LAPY_TRY((gemm_tn_blk<2, 8>(X, na, Y, act)));
-    } else if (blk && nb == 4) {
-      LAPY_TRY((gemm_tn_blk<4, 2>(X, na, Y, act)));
-    } else if (blk && nb == 8) {
-      LAPY_TRY((gemm_tn_blk<8, 1>(X, na, Y, act)));
+    if (X.bs == nb && Y.bs == nb && Y.bst == 0 && na == nb && (nb == 1 || nb == 2 || nb == 4 || nb == 8)) {
+      auto kern = nb == 1 ? gram_f64_kernel<1, 1> : nb == 2 ? gram_f64_kernel<2, 1>
+                          : nb == 4 ? gram_f64_kernel<4, 2> : gram_f64_kernel<8, 4>;
+      kern<<<P.gt.nchunk, 256, 0, st>>>(X.base, Y.base, P.gt.chunk_row, P.gt.chunk_seg, act, e.partial);
+      LAPY_TRY(lapy_check_launch("gram_f64_kernel"));
     } else {
       dim3 grid(P.gt.nchunk, lapy_ceil_div(na, kTile), lapy_ceil_div(nb, kTile));
       gemm_tn_partial_kernel<<<grid, 256, 0, st>>>(X, na, Y, nb, P.gt.chunk_row, P.gt.chunk_seg, act, e.partial);
       LAPY_TRY(lapy_check_launch("gemm_tn_partial_kernel"));
     }
-    dim3 g2(P.nseg, std::max(1u, std::min(64u, lapy_ceil_div((int64_t)na * nb, 256))));
-    gemm_tn_reduce_kernel<<<g2, 256, 0, st>>>(e.partial, na, nb, P.gt.seg_chunk, out, out_stride, ldo);
+    gemm_tn_reduce_kernel<<<reduce_grid(na, nb), 256, 0, st>>>(e.partial, na, nb, P.gt.seg_chunk, out, out_stride, ldo);
     return lapy_check_launch("gemm_tn_reduce_kernel");
   }
   // CGS products against basis blocks 0..nbasis/p-1 from the double-float copy
-  template <int PB, int JB>
+  template <int PB, int TPR, int JB>
   int gemm_tn_df_p(int nbasis, const double* Y, const int32_t* act) const {
     const int nblk = nbasis / PB;
     // Y split into (hi, lo) pairs once, not once per basis-block CTA (the
@@ -960,22 +1035,22 @@ struct EigOps {
     const int64_t m = P.n * PB;
     to_df_kernel<<<lapy_ceil_div(m, 256), 256, 0, st>>>(m, Y, e.MW_df);
     LAPY_TRY(lapy_check_launch("to_df_kernel"));
-    dim3 grid(P.gt.nchunk, lapy_ceil_div(nblk, JB));
-    gemm_tn_df_kernel<PB, JB><<<grid, 256, 0, st>>>(e.basis_df, P.n * PB, nblk, e.MW_df, P.gt.chunk_row,
-                                                    P.gt.chunk_seg, act, e.partial);
+    dim3 grid(P.tt.nchunk, lapy_ceil_div(nblk, JB));
+    gemm_tn_df_kernel<PB, TPR, JB><<<grid, 256, 0, st>>>(e.basis_df, P.n * PB, nblk, e.MW_df, P.tt.chunk_row,
+                                                         P.tt.chunk_seg, act, e.partial);
     return lapy_check_launch("gemm_tn_df_kernel");
   }
   int cgs_tn(int nbasis, const double* MW, double* out, int64_t out_stride, int ldo, const int32_t* act) const {
     const int p = P.p;
     int st_ = LAPY_ERR_INVALID;
-    if (p == 1) st_ = gemm_tn_df_p<1, 16>(nbasis, MW, act);
-    else if (p == 2) st_ = gemm_tn_df_p<2, 8>(nbasis, MW, act);
-    else if (p == 4) st_ = gemm_tn_df_p<4, 1>(nbasis, MW, act);
-    else if (p == 8) st_ = gemm_tn_df_p<8, 1>(nbasis, MW, act);
+    if (p == 1) st_ = gemm_tn_df_p<1, 1, 16>(nbasis, MW, act);
+    else if (p == 2) st_ = gemm_tn_df_p<2, 1, 4>(nbasis, MW, act);
+    else if (p == 4) st_ = gemm_tn_df_p<4, 1, 1>(nbasis, MW, act);
+    else if (p == 8) st_ = gemm_tn_df_p<8, 4, 1>(nbasis, MW, act);
     else return gemm_tn(BMat{e.basis, p, P.n * p}, nbasis, BMat{MW, p, 0}, p, out, out_stride, ldo, act);
     LAPY_TRY(st_);
-    dim3 g2(P.nseg, std::max(1u, std::min(64u, lapy_ceil_div((int64_t)nbasis * p, 256))));
-    gemm_tn_reduce_kernel<<<g2, 256, 0, st>>>(e.partial, nbasis, p, P.gt.seg_chunk, out, out_stride, ldo);
+    gemm_tn_reduce_kernel<<<reduce_grid(nbasis, p), 256, 0, st>>>(e.partial, nbasis, p, P.tt.seg_chunk, out,
+                                                                  out_stride, ldo);
     return lapy_check_launch("gemm_tn_reduce_kernel");
   }
   // (on the PCG's short chunks: the NN product has no per-chunk reduction,
@@ -1032,7 +1107,7 @@ struct EigOps {
       BMat MWm{e.MW, p, 0};
       LAPY_TRY(gemm_tn(Wm, p, MWm, p, e.G, (int64_t)p * p, p, e.active));
       double* R = pass == 0 ? e.R1 : e.R2;
-      chol_small_kernel<<<lapy_ceil_div(P.nseg, 64), 64, 0, st>>>(P.nseg, p, e.G, R, e.active, e.fail);
+      chol_small_kernel<<<lapy_ceil_div(P.nseg, 2), 64, 0, st>>>(P.nseg, p, e.G, R, e.active, e.fail);
       LAPY_TRY(lapy_check_launch("chol_small_kernel"));
       LAPY_TRY(launch_trsm_right(W, p, R, P.gt, st));
     }
@@ -1121,11 +1196,13 @@ static int eigs_run(const EigPlan& P, const EigPtrs& e, const int32_t* indptr, c
   std::vector<int32_t> lab;
   if (reorder) LAPY_TRY(reorder_system(P, e, &indptr, &indices, &a_vals, &m_vals, m_is_diag, &lab, st));
   EigOps ops{P, e, indptr, indices, a_vals, m_vals, m_is_diag, G, st, SellMatrix<double>()};
-  ChunkTable ct = P.ct, gt = P.gt;
+  ChunkTable ct = P.ct, gt = P.gt, tt = P.tt;
   LAPY_TRY(upload_chunk_table(&ct, e.ct_mem, st));
   LAPY_TRY(upload_chunk_table(&gt, e.gt_mem, st));
+  LAPY_TRY(upload_chunk_table(&tt, e.tt_mem, st));
   const_cast<EigPlan&>(P).ct = ct;
   const_cast<EigPlan&>(P).gt = gt;
+  const_cast<EigPlan&>(P).tt = tt;
 
   // K = A - sigma M (f64 and f32), Jacobi diagonal
   LAPY_TRY(lapy_csr_diag_index(n, indptr, indices, e.diag_pos, st));
@@ -1338,7 +1415,7 @@ static int eigs_run(const EigPlan& P, const EigPtrs& e, const int32_t* indptr, c
   }
   {
     dim3 grid(P.gt.nchunk, lapy_ceil_div(keff, 64), lapy_ceil_div(keff, 64));
-    dim3 g2(P.nseg, std::max(1u, std::min(64u, lapy_ceil_div((int64_t)keff * keff, 256))));
+    const dim3 g2 = ops.reduce_grid(keff, keff);
     gemm_tn_df_tile_kernel<<<grid, 256, 0, st>>>(e.X_df, keff, reinterpret_cast<const float2*>(e.AX), keff,
                                                  P.gt.chunk_row, e.partial);
     LAPY_TRY(lapy_check_launch("gemm_tn_df_tile_kernel"));
