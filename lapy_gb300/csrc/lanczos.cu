@@ -256,7 +256,7 @@ __device__ __forceinline__ int f64_lane_totals(double (&v)[NV], int& left) {
 // the sums over lanes cost 14 exchanges; one lane per row had 64 accumulators
 // and 320).  A warp's lanes read consecutive 16-byte pieces of X.  Bound by
 // the FP32 pipe (about 10 instructions per product) on large batches, by
-// latency on one mesh; per product 300 -> 11 us at 10,242 rows, 8 columns,
+// latency on one mesh; per product 300 -> 15 us at 10,242 rows, 8 columns,
 // 128 basis vectors.
 template <int P, int TPR, int JB>
 __global__ void __launch_bounds__(256) gemm_tn_df_kernel(const float2* __restrict__ X, int64_t bst, int nblk,

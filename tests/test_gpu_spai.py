@@ -168,3 +168,49 @@ def test_learned_heat_matches_oracle(cuda_ok):
             assert np.sqrt(np.sum(md * (x - ref) ** 2) / np.sum(md * ref ** 2)) <= 1e-8
     with pytest.raises(ValueError, match="precond"):
         heat.diffusion(ms[0], 0, precond="ilu")
+
+
+@pytest.mark.parametrize("ne", [1, 15, 16, 17, 63, 64, 65, 128, 64 * 304 - 1, 64 * 304 + 65])
+def test_backward_at_the_edges_of_tiles(cuda_ok, ne):
+    """Parameter gradient against 64 bits at partial and whole tiles of 64
+    edges, and where a CTA takes a second tile (304 CTAs resident)."""
+    import torch
+
+    from lapy_gb300.spai import SpaiNet
+
+    rng = np.random.default_rng(ne)
+    theta = ospai.init_params(3)
+    theta[-65:] = (rng.standard_normal(65) * 0.3).astype(np.float32)
+    feat = rng.standard_normal((ne, 6)).astype(np.float32)
+    dw = rng.standard_normal(ne).astype(np.float32)
+    net = SpaiNet(theta)
+    got = net.backward(torch.from_numpy(feat).cuda(), torch.from_numpy(dw).cuda(), 0.5).cpu().numpy()
+
+    P = {k: np.asarray(v, np.float64) for k, v in ospai.unpack(ospai.bf16(theta)).items()}
+    W1, W2, W3 = (P[k].reshape(s) for k, s in (("W1", (64, 6)), ("W2", (64, 64)), ("W3", (64,))))
+    f, d = feat.astype(np.float64), dw.astype(np.float64)[:, None]
+    h1 = np.tanh(f @ W1.T + P["b1"].ravel())
+    h2 = np.tanh(h1 @ W2.T + P["b2"].ravel())
+    # bounds in units of 2^-24: every value with its error, sums of m terms
+    # with m roundings; tanh within 4; products of split factors within 4
+    u = 2.0**-24
+    z1 = np.abs(f) @ np.abs(W1).T + np.abs(P["b1"].ravel())
+    e1 = 8 * u * z1 + 4 * u
+    z2 = np.abs(h1) @ np.abs(W2).T + np.abs(P["b2"].ravel())
+    e2 = e1 @ np.abs(W2).T + 200 * u * z2 + 4 * u
+    dz2, a2 = d * W3 * (1 - h2**2), np.abs(d * W3)
+    b2 = a2 * (2 * e2 + 8 * u)
+    s1, a1 = dz2 @ W2, a2 @ np.abs(W2)
+    dz1 = s1 * (1 - h1**2)
+    b1 = b2 @ np.abs(W2) + a1 * (200 * u + 2 * e1)
+    terms = 64 * 6 + -(-ne // 64) + 16  # roundings on the way of one term
+    want, tol = {}, {}
+    want["W1"], tol["W1"] = dz1.T @ f, b1.T @ np.abs(f) + terms * u * (a1.T @ np.abs(f))
+    want["b1"], tol["b1"] = dz1.sum(0), b1.sum(0) + terms * u * a1.sum(0)
+    want["W2"], tol["W2"] = dz2.T @ h1, (b2.T @ np.abs(h1) + a2.T @ e1) + terms * u * (a2.T @ np.abs(h1))
+    want["b2"], tol["b2"] = dz2.sum(0), b2.sum(0) + terms * u * a2.sum(0)
+    want["W3"], tol["W3"] = (d * h2).sum(0), (np.abs(d) * (e2 + terms * u * np.abs(h2))).sum(0)
+    want["b3"], tol["b3"] = d.sum(), terms * u * np.abs(d).sum()
+    ref = 0.5 * np.concatenate([np.ravel(want[k]) for k, _ in ospai.LAYOUT])
+    bound = 0.5 * np.concatenate([np.ravel(tol[k]) for k, _ in ospai.LAYOUT])
+    assert np.all(np.abs(got - ref) <= bound + 1e-30)
