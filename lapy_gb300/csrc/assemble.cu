@@ -9,12 +9,14 @@
 
 namespace lapy {
 
-// Local slots in the reference's COO order (i and j of slots 0, 1, ...).
+// COO slot of the local entry (i, j), four bits each, in the reference's order
 // Triangles: solver.py:174-175  (t1,t2,t2,t3,t3,t1,t1,t2,t3) x (t2,t1,t3,t2,t1,t3,t1,t2,t3)
 // Tetrahedra: solver.py:492-497.
-// COO slot of the local entry (i, j).
-__constant__ int8_t kTriaL[9] = {6, 0, 5, 1, 7, 2, 4, 3, 8};
-__constant__ int8_t kTetL[16] = {12, 0, 5, 6, 1, 13, 2, 8, 4, 3, 14, 10, 7, 9, 11, 15};
+template <int NPE>
+__device__ __forceinline__ int coo_slot(int i, int j) {
+  constexpr uint64_t kSlots = NPE == 3 ? 0x834271506ull : 0xfb97ae3482d1650cull;
+  return (int)(kSlots >> (4 * (i * NPE + j))) & 15;
+}
 
 // ---------------------------------------------------------------------------
 // Symbolic phase
@@ -27,7 +29,7 @@ struct SymbolicWs {
   int32_t* corner_ptr;  // n + 1  exclusive scan of row_count
   int32_t* row_nnz;     // n      distinct columns per row
   int32_t* corners;     // m*npe  corners, bucketed by row
-  uint64_t* sorted;     // m*L    keys (col << 32 | pos) sorted inside each row
+  uint64_t* sorted;     // m*L    keys (col << 32 | pos) sorted inside each row, bit 31: first of its column
   int32_t* scan_scratch;
   int* bad;             // set if an index lies outside [0, n)
 };
@@ -91,7 +93,7 @@ template <int NPE>
 __device__ __forceinline__ uint64_t coo_key(const int32_t* __restrict__ elems, const int32_t* __restrict__ cs, int a) {
   const int32_t c = cs[a / NPE];
   const int j = a % NPE, e = c / NPE, i = c - e * NPE;
-  const int l = NPE == 3 ? kTriaL[i * NPE + j] : kTetL[i * NPE + j];
+  const int l = coo_slot<NPE>(i, j);
   return ((uint64_t)(uint32_t)elems[(int64_t)e * NPE + j] << 32) | (uint32_t)(e * (NPE * NPE) + l);
 }
 
@@ -137,76 +139,210 @@ __device__ __forceinline__ void rank_chunk(const int32_t* __restrict__ elems, co
   __syncwarp();
 }
 
-// Warp per row: rank sort of the row's keys (unique, so the rank of a key is
-// the number of smaller keys), then count distinct columns.  Bound by the
-// shared-memory reads of the rank loop; a row's keys are formed from its
-// corners on the way in, so that no key list is bucketed through memory (8
-// bytes and one atomic per entry before, now 4 bytes and one per corner).
-// At 1.25 million rows and 22.4 million entries counting and bucketing went
-// from 286 to 59 us, the sort from 374 to 519 us.
+constexpr uint32_t kFirst = 0x80000000u;  // positions are below 2^31
+
+// One warp sorts a row of k keys by rank (the keys are unique, so the rank of
+// a key is the number of smaller keys), marks the first key of every column
+// and returns the number of columns.
 template <int NPE>
-__global__ void __launch_bounds__(32 * kSortWarps) row_sort_kernel(int64_t n, const int32_t* __restrict__ elems,
-                                                                   const int32_t* __restrict__ corner_ptr,
-                                                                   const int32_t* __restrict__ corners,
-                                                                   uint64_t* __restrict__ sorted,
-                                                                   int32_t* __restrict__ row_nnz) {
-  __shared__ uint64_t keys[kSortWarps][kSortChunk];
-  const int lane = threadIdx.x & 31;
-  const int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (row >= n) return;
-  uint64_t* sm = keys[threadIdx.x >> 5];
-  const int32_t c0 = corner_ptr[row];
-  const int k = (corner_ptr[row + 1] - c0) * NPE;
-  const int32_t* cs = corners + c0;
-  uint64_t* out = sorted + (int64_t)c0 * NPE;
+__device__ __forceinline__ int warp_sort_row(const int32_t* __restrict__ elems, const int32_t* __restrict__ cs, int k,
+                                             uint64_t* sm, uint64_t* __restrict__ out, int lane) {
   for (int a0 = 0; a0 < k; a0 += kSortChunk) {
     const int na = k - a0;
     if (na <= 32) rank_chunk<NPE, 1>(elems, cs, k, a0, lane, sm, out);
     else if (na <= 64) rank_chunk<NPE, 2>(elems, cs, k, a0, lane, sm, out);
     else rank_chunk<NPE, 4>(elems, cs, k, a0, lane, sm, out);
   }
-  // distinct columns: entries whose column differs from the previous entry
-  const bool kept = k <= kSortChunk;
   int cnt = 0;
-  for (int a = lane; a < k; a += 32) {
-    const uint64_t key = kept ? sm[a] : out[a];
-    const bool first = a == 0 || (uint32_t)((kept ? sm[a - 1] : out[a - 1]) >> 32) != (uint32_t)(key >> 32);
-    if (kept) out[a] = key;
-    cnt += first ? 1 : 0;
+  if (k <= kSortChunk) {
+    for (int a = lane; a < k; a += 32) {
+      const uint64_t key = sm[a];
+      const bool first = a == 0 || (uint32_t)(sm[a - 1] >> 32) != (uint32_t)(key >> 32);
+      out[a] = first ? key | kFirst : key;
+      cnt += first ? 1 : 0;
+    }
+  } else {
+    uint32_t* half = reinterpret_cast<uint32_t*>(out);  // column at 2a + 1, position at 2a
+    for (int a = lane; a < k; a += 32) {
+      const bool first = a == 0 || half[2 * (int64_t)a - 1] != half[2 * (int64_t)a + 1];
+      if (first) half[2 * (int64_t)a] |= kFirst;
+      cnt += first ? 1 : 0;
+    }
   }
-  cnt = warp_sum(cnt);
-  if (lane == 0) row_nnz[row] = cnt;
+  __syncwarp();
+  return warp_sum(cnt);
 }
 
-// Warp per row: write column indices, run starts and source positions.
-__global__ void row_fill_kernel(int64_t n, int npe, int64_t nnz, const int32_t* __restrict__ corner_ptr,
-                                const uint64_t* __restrict__ sorted,
-                                const int32_t* __restrict__ indptr, int32_t* __restrict__ indices,
-                                int32_t* __restrict__ seg_ptr, int32_t* __restrict__ seg_src) {
+// Tetrahedra: one warp per row (about 24 corners, 96 keys).
+__global__ void __launch_bounds__(32 * kSortWarps) row_sort_tet_kernel(int64_t n, const int32_t* __restrict__ elems,
+                                                                       const int32_t* __restrict__ corner_ptr,
+                                                                       const int32_t* __restrict__ corners,
+                                                                       uint64_t* __restrict__ sorted,
+                                                                       int32_t* __restrict__ row_nnz) {
+  __shared__ uint64_t keys[kSortWarps][kSortChunk];
   const int lane = threadIdx.x & 31;
   const int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (row >= n) return;
-  const int32_t b0 = npe * corner_ptr[row], b1 = npe * corner_ptr[row + 1];
-  const int k = b1 - b0;
-  if (row == n - 1 && lane == 0) seg_ptr[nnz] = b1;
-  int32_t out = indptr[row];
-  for (int base = 0; base < k; base += 32) {
-    const int a = base + lane;
-    bool first = false;
-    uint32_t col = 0;
-    if (a < k) {
-      const uint64_t key = sorted[b0 + a];
-      col = (uint32_t)(key >> 32);
-      first = (a == 0) || ((uint32_t)(sorted[b0 + a - 1] >> 32) != col);
-      seg_src[b0 + a] = (int32_t)(uint32_t)(key & 0xffffffffu);
+  const int32_t c0 = corner_ptr[row];
+  const int cnt = warp_sort_row<4>(elems, corners + c0, (corner_ptr[row + 1] - c0) * 4, keys[threadIdx.x >> 5],
+                                   sorted + (int64_t)c0 * 4, lane);
+  if (lane == 0) row_nnz[row] = cnt;
+}
+
+// Triangles: one thread per row of up to kNarrow corners, wider rows (and rows
+// of elements that name a vertex twice) by the warp afterwards.  A thread sorts
+// its corners and the two off-diagonal keys of each by networks in registers;
+// the diagonal entries follow from the corners' order.  A warp's rows are
+// neighbours in memory, so the keys leave through shared memory in whole
+// lines.  A warp per row was bound by instruction issue (about 400 slots for 18
+// keys): 374 us for 1.25 million rows with the keys from memory, 72 us now.
+constexpr int kNarrow = 8;
+constexpr int kTriaSortWarps = 4;
+
+template <typename K, int N>
+__device__ __forceinline__ void sort_network(K (&x)[N]) {  // Batcher's odd-even merge sort, N a power of two
+#pragma unroll
+  for (int p = 1; p < N; p *= 2)
+#pragma unroll
+    for (int k = p; k >= 1; k /= 2)
+#pragma unroll
+      for (int j = 0; j + k < N; ++j)
+        if (j >= k % p && (j - k % p) % (2 * k) < k && j / (2 * p) == (j + k) / (2 * p)) {
+          const K lo = min(x[j], x[j + k]), hi = max(x[j], x[j + k]);
+          x[j] = lo;
+          x[j + k] = hi;
+        }
+}
+
+__global__ void __launch_bounds__(32 * kTriaSortWarps) row_sort_tria_kernel(int64_t n,
+                                                                            const int32_t* __restrict__ elems,
+                                                                            const int32_t* __restrict__ corner_ptr,
+                                                                            const int32_t* __restrict__ corners,
+                                                                            uint64_t* __restrict__ sorted,
+                                                                            int32_t* __restrict__ row_nnz) {
+  __shared__ uint64_t stage[kTriaSortWarps][32 * kNarrow * 3];  // also the warp's kSortChunk keys
+  const int lane = threadIdx.x & 31;
+  const int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, row0 = row - lane;
+  if (row0 >= n) return;
+  uint64_t* sm = stage[threadIdx.x >> 5];
+  const int32_t c0 = row < n ? corner_ptr[row] : 0;
+  const int val = row < n ? corner_ptr[row + 1] - c0 : 0;
+  bool wide = val > kNarrow;
+  uint32_t c[kNarrow];
+  uint64_t key[2 * kNarrow];
+  if (!wide) {
+#pragma unroll
+    for (int d = 0; d < kNarrow; ++d) c[d] = d < val ? (uint32_t)corners[c0 + d] : 0xffffffffu;
+    sort_network(c);
+#pragma unroll
+    for (int d = 0; d < kNarrow; ++d) {
+      const uint32_t e = c[d] / 3, i = c[d] - 3 * e;
+#pragma unroll
+      for (uint32_t o = 0; o < 2; ++o) {
+        const uint32_t j = (i + 1 + o) % 3;
+        uint64_t x = ~uint64_t(0);
+        if (d < val) {
+          const uint32_t col = (uint32_t)elems[3 * (int64_t)e + j];
+          wide |= col == (uint32_t)row;
+          x = ((uint64_t)col << 32) | (9 * e + coo_slot<3>(i, j));
+        }
+        key[2 * d + o] = x;
+      }
     }
-    const unsigned mask = __ballot_sync(0xffffffffu, first);
-    if (first) {
-      const int rank = __popc(mask & ((1u << lane) - 1u));
-      indices[out + rank] = (int32_t)col;
-      seg_ptr[out + rank] = b0 + a;
+    sort_network(key);
+  }
+  const bool staged = !__any_sync(0xffffffffu, wide);
+  const int32_t w0 = __shfl_sync(0xffffffffu, c0, 0);
+  if (!wide && val > 0) {
+    uint64_t* out = staged ? sm + 3 * (c0 - w0) : sorted + 3 * (int64_t)c0;
+    int cnt = 1, less = 0;
+#pragma unroll
+    for (int q = 0; q < 2 * kNarrow; ++q)
+      if (q < 2 * val) {
+        const uint32_t col = (uint32_t)(key[q] >> 32);
+        const bool first = q == 0 || col != (uint32_t)(key[q - (q > 0)] >> 32), before = col < (uint32_t)row;
+        out[before ? q : q + val] = first ? key[q] | kFirst : key[q];
+        cnt += first ? 1 : 0;
+        less += before ? 1 : 0;
+      }
+#pragma unroll
+    for (int d = 0; d < kNarrow; ++d)
+      if (d < val) {
+        const uint32_t e = c[d] / 3, pos = 9 * e + 6 + (c[d] - 3 * e);
+        out[less + d] = ((uint64_t)(uint32_t)row << 32) | (d == 0 ? pos | kFirst : pos);
+      }
+    row_nnz[row] = cnt;
+  } else if (row < n && val == 0) {
+    row_nnz[row] = 0;
+  }
+  __syncwarp();
+  if (staged) {
+    const int total = 3 * (corner_ptr[min(row0 + 32, n)] - w0);
+    for (int t = lane; t < total; t += 32) sorted[3 * (int64_t)w0 + t] = sm[t];
+    return;
+  }
+  for (unsigned todo = __ballot_sync(0xffffffffu, wide); todo; todo &= todo - 1) {
+    const int src = __ffs(todo) - 1;
+    const int32_t r0 = __shfl_sync(0xffffffffu, c0, src);
+    const int k = 3 * __shfl_sync(0xffffffffu, val, src);
+    const int cnt = warp_sort_row<3>(elems, corners + r0, k, sm, sorted + 3 * (int64_t)r0, lane);
+    if (lane == 0) row_nnz[row0 + src] = cnt;
+  }
+}
+
+// Column indices, run starts and source positions: a CTA takes kFillRows rows,
+// whose entries and runs are contiguous, and compacts the marked keys.  Bound
+// by memory: 1.25 million rows 185 us with a warp per row, 51 us now.
+constexpr int kFillRows = 256;
+constexpr int kFillWarps = 8;
+constexpr int kFillItems = 4;
+
+__global__ void __launch_bounds__(32 * kFillWarps) row_fill_kernel(int64_t n, int npe, int64_t nnz,
+                                                                   const int32_t* __restrict__ corner_ptr,
+                                                                   const uint64_t* __restrict__ sorted,
+                                                                   const int32_t* __restrict__ indptr,
+                                                                   int32_t* __restrict__ indices,
+                                                                   int32_t* __restrict__ seg_ptr,
+                                                                   int32_t* __restrict__ seg_src) {
+  __shared__ int wsum[2][kFillWarps];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t r0 = (int64_t)blockIdx.x * kFillRows, r1 = min(r0 + kFillRows, n);
+  const int64_t b0 = (int64_t)npe * corner_ptr[r0], b1 = (int64_t)npe * corner_ptr[r1];
+  if (r1 == n && threadIdx.x == 0) seg_ptr[nnz] = (int32_t)b1;
+  int32_t out = indptr[r0];
+  int buf = 0;
+  for (int64_t base = b0; base < b1; base += 32 * kFillWarps * kFillItems, buf ^= 1) {
+    const int64_t a0 = base + (warp * kFillItems) * 32 + lane;
+    uint64_t key[kFillItems];
+    unsigned mask[kFillItems];
+    int cnt = 0;
+#pragma unroll
+    for (int q = 0; q < kFillItems; ++q) key[q] = a0 + 32 * q < b1 ? sorted[a0 + 32 * q] : 0;
+#pragma unroll
+    for (int q = 0; q < kFillItems; ++q) {
+      mask[q] = __ballot_sync(0xffffffffu, ((uint32_t)key[q] & kFirst) != 0);
+      cnt += __popc(mask[q]);
     }
-    out += __popc(mask);
+    if (lane == 0) wsum[buf][warp] = cnt;
+    __syncthreads();  // the other buffer's readers are past the next iteration's barrier
+    int32_t at = out;
+#pragma unroll
+    for (int w = 0; w < kFillWarps; ++w) {
+      const int x = wsum[buf][w];
+      at += w < warp ? x : 0;
+      out += x;
+    }
+#pragma unroll
+    for (int q = 0; q < kFillItems; ++q) {
+      const int64_t a = a0 + 32 * q;
+      if (a < b1) seg_src[a] = (int32_t)((uint32_t)key[q] & ~kFirst);
+      if ((uint32_t)key[q] & kFirst) {
+        const int32_t o = at + __popc(mask[q] & ((1u << lane) - 1u));
+        indices[o] = (int32_t)(key[q] >> 32);
+        seg_ptr[o] = (int32_t)a;
+      }
+      at += __popc(mask[q]);
+    }
   }
 }
 
@@ -597,11 +733,12 @@ extern "C" int lapy_csr_symbolic_count(const int32_t* elems, int64_t m, int npe,
   corner_bucket_kernel<<<lapy_ceil_div(nc, 256), 256, 0, stream>>>(elems, nc, ws.corner_ptr, ws.row_count,
                                                                    ws.corners, n);
   LAPY_TRY(lapy_check_launch("corner_bucket_kernel"));
-  const unsigned rb = lapy_ceil_div(n, kSortWarps);
   if (npe == 3)
-    row_sort_kernel<3><<<rb, 32 * kSortWarps, 0, stream>>>(n, elems, ws.corner_ptr, ws.corners, ws.sorted, ws.row_nnz);
+    row_sort_tria_kernel<<<lapy_ceil_div(n, 32 * kTriaSortWarps), 32 * kTriaSortWarps, 0, stream>>>(
+        n, elems, ws.corner_ptr, ws.corners, ws.sorted, ws.row_nnz);
   else
-    row_sort_kernel<4><<<rb, 32 * kSortWarps, 0, stream>>>(n, elems, ws.corner_ptr, ws.corners, ws.sorted, ws.row_nnz);
+    row_sort_tet_kernel<<<lapy_ceil_div(n, kSortWarps), 32 * kSortWarps, 0, stream>>>(
+        n, elems, ws.corner_ptr, ws.corners, ws.sorted, ws.row_nnz);
   LAPY_TRY(lapy_check_launch("row_sort_kernel"));
   LAPY_TRY(exclusive_scan_i32(ws.row_nnz, indptr, n, ws.scan_scratch, stream));
   // one wait for both results (a bad index is left out of the buckets above)
@@ -630,7 +767,7 @@ extern "C" int lapy_csr_symbolic_fill(const int32_t* elems, int64_t m, int npe, 
   SymbolicWs ws;
   char* base = (char*)(((uintptr_t)workspace + 255) & ~uintptr_t(255));
   symbolic_layout(n, m, npe, base, &ws);
-  row_fill_kernel<<<lapy_ceil_div(n * 32, 256), 256, 0, stream>>>(n, npe, nnz, ws.corner_ptr, ws.sorted, indptr,
+  row_fill_kernel<<<lapy_ceil_div(n, kFillRows), 32 * kFillWarps, 0, stream>>>(n, npe, nnz, ws.corner_ptr, ws.sorted, indptr,
                                                                   indices, seg_ptr, seg_src);
   return lapy_check_launch("row_fill_kernel");
 }

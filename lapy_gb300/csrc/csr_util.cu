@@ -90,9 +90,8 @@ __global__ void edge_len_final_kernel(const double* psum, const long long* pcnt,
 
 // Mean edge length of a segment's strict upper triangle: a cluster of CTAs per
 // segment, thread-strided rows, sums in a fixed order (block_sum, then the
-// CTAs by rank).  Bound by the latency of the gathers, so a segment takes
-// eight CTAs; 256 meshes of 9,740 rows: 738 us
-// with one, 392 us now (FP64 rate).
+// CTAs by rank).  Eight CTAs per segment, as one is bound by the latency of its
+// gathers: 256 meshes of 9,740 rows 738 us with one, 392 us now (FP64 rate).
 constexpr int kSegCtas = 8;
 
 template <typename T>
@@ -103,6 +102,7 @@ __global__ void __cluster_dims__(kSegCtas, 1, 1)
   __shared__ double sh[32];
   __shared__ double part[kSegCtas], cnt[kSegCtas];  // of rank 0: the CTAs' sums
   const int s = blockIdx.x / kSegCtas, rank = blockIdx.x % kSegCtas;
+  cl_sync(kSegCtas);  // every CTA runs before the first remote store
   double acc = 0.0;
   int cn = 0;
   for (int64_t r = (int64_t)seg_row[s] + rank * blockDim.x + threadIdx.x; r < seg_row[s + 1];

@@ -94,6 +94,35 @@ def test_degenerate_elements(cuda_ok, npe, lump):
         assert np.all(np.abs(g - want) <= (len(t) + 16) * 2.0**-53 * size)
 
 
+@pytest.mark.parametrize("npe", [3, 4])
+def test_elements_that_name_a_vertex_twice(cuda_ok, npe):
+    v, t = _fan(30, npe, seed=8)
+    t[4, 1] = t[4, 0]
+    t[9, 2] = t[9, 0]
+    ptr, idx, refs = _reference(v, t, False, np.float64)
+    pat, *got = _device(v, t, False, False)
+    np.testing.assert_array_equal(pat.indptr.cpu().numpy(), ptr)
+    np.testing.assert_array_equal(pat.indices.cpu().numpy(), idx)
+    for (want, size), g in zip(refs, got):  # clamped elements as above
+        assert np.all(np.abs(g - want) <= (len(t) + 16) * 2.0**-53 * size)
+
+
+def test_many_rows(cuda_ok):
+    """Rows of 6 corners in whole warps and CTAs, and a wide row among narrow ones."""
+    from lapy_gb300 import meshes
+
+    m = meshes.icosphere(5)
+    v, t = np.asarray(m.v, np.float64), np.asarray(m.t, np.int32)
+    fv, ft = _fan(100, 3, seed=2)
+    v, t = np.r_[v, fv, v], np.r_[t, ft + len(v), t + len(v) + len(fv)].astype(np.int32)
+    ptr, idx, ((a, _), (mm, _)) = _reference(v, t, False, np.float64)
+    pat, ga, gm = _device(v, t, False, False)
+    np.testing.assert_array_equal(pat.indptr.cpu().numpy(), ptr)
+    np.testing.assert_array_equal(pat.indices.cpu().numpy(), idx)
+    np.testing.assert_array_equal(ga, a)
+    np.testing.assert_array_equal(gm, mm)
+
+
 def test_out_of_range_index_is_refused(cuda_ok):
     import torch
 
