@@ -306,11 +306,13 @@ __global__ void spai_gather_kernel(int64_t m, const int32_t* __restrict__ umap, 
 // shared memory; then every warp accumulates 16 rows of dW2 = dz2' h1 and of
 // [dW1 | db1] = dz1' [f | 1] over the CTA's 64 edges in registers.  Activations
 // and gradients are split into three BF16 terms (about 24 bits), products of
-// two split factors keep the six terms above 2^-24.  Against 64 bits on the
-// same FP32 inputs the gradient is off by 1.5e-7 (geometric mean over 24
-// batches of 46,000 to 912,000 entries), 2.8e-7 for the FP32 path it replaces
-// (one thread per edge, one thread per group of parameters), which took 1,054
-// us for 462,000 entries, 11 TFLOP/s.  Whole gradient pass: 1,194 -> 383 us.
+// two split factors keep the six terms above 2^-24, and the 16-wide products
+// of a sum are added in FP32 (the tensor pipe rounds its running sums towards
+// zero).  Against 64 bits on the same FP32 inputs the gradient is off by 7.4e-8
+// (geometric mean over 24 batches of 46,000 to 912,000 entries), 2.8e-7 for the
+// FP32 path it replaces (one thread per edge, one thread per group of
+// parameters), which took 1,054 us for 462,000 entries, 11 TFLOP/s.  Whole
+// gradient pass there: 1,192 -> 364 us, off by 6.40e-6, before 6.42e-6.
 constexpr int kBwdWarps = 4;
 constexpr int kBwdThreads = 32 * kBwdWarps;
 constexpr int kBwdEdges = 16 * kBwdWarps;
@@ -429,9 +431,12 @@ __global__ void __launch_bounds__(kBwdThreads, 2) spai_backward_kernel(int64_t n
       for (int t = 0; t < 4; ++t) {
         const uint32_t b0 = W2w[(n * kW2Ld + 16 * t + 2 * tig) >> 1];
         const uint32_t b1 = W2w[(n * kW2Ld + 16 * t + 8 + 2 * tig) >> 1];
-        mma_bf16_16816(acc, a1[2][t], b0, b1);
-        mma_bf16_16816(acc, a1[1][t], b0, b1);
-        mma_bf16_16816(acc, a1[0][t], b0, b1);
+        float hi[4] = {0.f, 0.f, 0.f, 0.f};
+        mma_bf16_16816(hi, a1[2][t], b0, b1);
+        mma_bf16_16816(hi, a1[1][t], b0, b1);
+        mma_bf16_16816(hi, a1[0][t], b0, b1);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[c] += hi[c];
       }
       const int u = 8 * j + 2 * tig;
       float z[4];
@@ -464,9 +469,12 @@ __global__ void __launch_bounds__(kBwdThreads, 2) spai_backward_kernel(int64_t n
       for (int t = 0; t < 4; ++t) {
         const uint32_t b0 = W2Tw[(n * kW2Ld + 16 * t + 2 * tig) >> 1];
         const uint32_t b1 = W2Tw[(n * kW2Ld + 16 * t + 8 + 2 * tig) >> 1];
-        mma_bf16_16816(acc, a2[2][t], b0, b1);
-        mma_bf16_16816(acc, a2[1][t], b0, b1);
-        mma_bf16_16816(acc, a2[0][t], b0, b1);
+        float hi[4] = {0.f, 0.f, 0.f, 0.f};
+        mma_bf16_16816(hi, a2[2][t], b0, b1);
+        mma_bf16_16816(hi, a2[1][t], b0, b1);
+        mma_bf16_16816(hi, a2[0][t], b0, b1);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[c] += hi[c];
       }
       const int u = 8 * j + 2 * tig;
 #pragma unroll
