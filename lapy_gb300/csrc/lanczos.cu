@@ -975,7 +975,7 @@ static size_t layout_eig(const EigPlan& P, char* base, EigPtrs* q) {
   e.wn0 = (double*)take(8 * (size_t)ns * p);
   e.wn1 = (double*)take(8 * (size_t)ns * p);
   e.active2 = (int32_t*)take(4 * ns);
-  e.rcnt = (unsigned long long*)take(16);
+  e.rcnt = (unsigned long long*)take(32);  // two counters, then the StepStatus of a block step
   const bool reorder = P.precond == kPrecTwoLevel;
   e.perm = (int32_t*)take(reorder ? 4 * n : 0);
   e.iperm = (int32_t*)take(reorder ? 4 * n : 0);
@@ -1116,20 +1116,58 @@ struct EigOps {
   }
 };
 
-// Cost model of the convergence-check stride (seconds on this part): a dense
-// eigensolve of an m x m projected matrix per CTA, in waves of one CTA per SM;
-// a block step's fixed cost plus its PCG iterations (grid-barrier latency and
-// rows streamed).
-constexpr double kCheckSecPerCube = 2.0e-9;
-constexpr double kStepSec = 1.0e-3;
-constexpr double kIterSec = 2.0e-5;
-constexpr double kIterSecPerRow = 9.0e-11;
+// Cost model of the convergence-check stride (seconds on this part): a check of
+// m x m projected matrices (1.0 ms at m = 128, 2.1 ms at 224 for one mesh, 3.1
+// ms at 160 for 128 meshes); a block step's fixed cost plus its inner
+// iterations, on chip (0.8 ms at 10,242 rows and 110 iterations, 2.3 ms at
+// 244,228, 10 ms at 1,251,846) or as grid-wide launches.
+constexpr double kCheckSecPerDim = 1.0e-5;
+constexpr double kCheckMeshes = 64.0;  // meshes that double a check's time
+constexpr double kChipStepSec = 3.5e-4, kChipIterSec = 4.0e-6, kChipIterSecPerRow = 6.0e-11;
+constexpr double kGridStepSec = 1.0e-3, kGridIterSec = 2.0e-5, kGridIterSecPerRow = 9.0e-11;
+// Pairs that converge per basis vector once the first check is made: 0.33 to
+// 0.37 measured for 50 pairs (10,242-vertex sphere, batches of 24 and 128
+// meshes), 0.16 for 10 pairs.
+constexpr double kPairsPerVector = 0.35;
 
 // Threshold of the selective second Gram-Schmidt pass (reorth_mask_kernel):
 // the classical 1/sqrt(2).  On the batched ShapeDNA workload about 98 % of the
 // (mesh, block step) pairs still repeat the pass; a threshold of 1e-2 skipped
 // 98 % of them but slowed Lanczos convergence (more steps, unconverged meshes).
 constexpr double kReorthEta = 0.7071067811865476;
+
+// What the host needs to know of a block step, in one small copy: the first
+// status that is not LAPY_OK among the inner solve's columns, its iterations,
+// and whether a Cholesky of an active segment failed.
+struct StepStatus {
+  long long iters;
+  int32_t status, fail;
+};
+
+__global__ void step_status_kernel(int nsp, const int32_t* __restrict__ state,
+                                   const unsigned long long* __restrict__ ctl, int ns,
+                                   const int32_t* __restrict__ fail, const int32_t* __restrict__ active,
+                                   StepStatus* __restrict__ out) {
+  __shared__ int first, any;
+  if (threadIdx.x == 0) {
+    first = INT_MAX;
+    any = 0;
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < nsp; i += blockDim.x)
+    if (state[i] != LAPY_OK) {
+      atomicMin(&first, i);
+      break;
+    }
+  for (int s = threadIdx.x; s < ns; s += blockDim.x)
+    if (active[s] && fail[s]) any = 1;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    out->iters = (long long)ctl[0];
+    out->status = first < INT_MAX ? state[first] : LAPY_OK;
+    out->fail = any;
+  }
+}
 
 struct EigResult {
   std::vector<int32_t> status;
@@ -1264,18 +1302,27 @@ static int eigs_run(const EigPlan& P, const EigPtrs& e, const int32_t* indptr, c
   res->status.assign(ns, LAPY_ERR_NOCONV);
   res->nbasis.assign(ns, 0);
   // First check once the basis holds ~2.5 k vectors (shift-invert Lanczos
-  // needs 3-5 k); afterwards the stride is the larger of (a) the gap to k
-  // converged pairs and (b) the stride that balances the cost of a check c
-  // against that of a block step s: checking every m steps costs c/m per step
-  // and overshoots convergence by (m-1)/2 steps on average, least at
-  // m = sqrt(2 c / s).  c and s come from a cost model of this GPU (fitted
-  // to measured dense-eigensolver and PCG times), not from timers, so the
-  // stopping step - and with it every result - is the same on every run.
+  // needs 3-5 k); afterwards the stride is the larger of (a) the block steps
+  // that the missing pairs take, on the mean over the unconverged meshes, and
+  // (b) the stride that balances the cost of a check c against that of a block
+  // step s: checking every m steps costs c/m per step and overshoots
+  // convergence by (m-1)/2 steps on average, least at m = sqrt(2 c / s).  c and
+  // s come from a cost model of this GPU, not from timers, so the stopping
+  // step - and with it every result - is the same on every run.  (With half of
+  // the missing pairs' blocks as (a), 10 checks instead of 5 for 642 vertices
+  // and 11 instead of 6 for 128 meshes.)
   const int first_check = std::max((keff + p + p - 1) / p, (int)std::ceil(2.5 * k / p));
   int next_check = first_check;
   int64_t step_pcg_iters = 0;
-  const int sms = lapy_num_sms();
   std::vector<int32_t> hnconv(ns);
+  auto inner_done = [&](int status, int64_t iters) -> int {
+    res->inner_iters += iters;
+    step_pcg_iters = iters;
+    if (status != LAPY_ERR_NAN && status != LAPY_ERR_BREAKDOWN) return LAPY_OK;
+    lapy_set_last_message("eigs: inner solve failed (%s)", lapy_status_string(status));
+    return status;
+  };
+  StepStatus* dstat = (StepStatus*)(e.rcnt + 2);
   int j = 0;
   bool all_done = false;
   std::vector<int32_t> seg_conv_blocks(ns, 0);
@@ -1286,14 +1333,16 @@ static int eigs_run(const EigPlan& P, const EigPtrs& e, const int32_t* indptr, c
     LAPY_TRY(ops.apply_M(Qj, e.Y, p));
     zero_inactive_kernel<<<P.ct.nchunk, 256, 0, st>>>(e.Y, p, P.ct.chunk_row, P.ct.chunk_seg, e.active);
     LAPY_TRY(lapy_check_launch("zero_inactive_kernel"));
-    IrStats irs;
-    LAPY_TRY(ir_solve(K, P.ct, p, e.Y, e.W, inner_rtol, inner_maxiter, 1, round_rtol, 16, e.ir_ws, e.ir_bytes,
-                      st, &irs, nullptr, nullptr));
-    res->inner_iters += irs.pcg_iters;
-    step_pcg_iters = irs.pcg_iters;
-    if (irs.status == LAPY_ERR_NAN || irs.status == LAPY_ERR_BREAKDOWN) {
-      lapy_set_last_message("eigs: inner solve failed (%s)", lapy_status_string(irs.status));
-      return irs.status;
+    // the solve's status is read with the step's at its end: a wait here left
+    // the GPU idle for the launches of the rest of the step
+    IrDeferred def;
+    LAPY_TRY(ir_solve_deferred(K, P.ct, p, e.Y, e.W, inner_rtol, inner_maxiter, round_rtol, 16, e.ir_ws, e.ir_bytes,
+                               st, &def));
+    if (!def.taken) {
+      IrStats irs;
+      LAPY_TRY(ir_solve(K, P.ct, p, e.Y, e.W, inner_rtol, inner_maxiter, 1, round_rtol, 16, e.ir_ws, e.ir_bytes, st,
+                        &irs, nullptr, nullptr));
+      LAPY_TRY(inner_done(irs.status, irs.pcg_iters));
     }
     // classical Gram-Schmidt against the basis blocks 0..j in the M inner
     // product: a first pass, then a second one where the first cancelled
@@ -1318,12 +1367,22 @@ static int eigs_run(const EigPlan& P, const EigPtrs& e, const int32_t* indptr, c
     LAPY_CUDA_TRY(cudaMemcpyAsync(Qn, e.W, 8 * n * p, cudaMemcpyDeviceToDevice, st));
     LAPY_TRY(ops.chol_qr2(Qn));
     LAPY_TRY(ops.basis_to_df(j + 1));
-    LAPY_CUDA_TRY(cudaMemcpyAsync(hfail.data(), e.fail, 4 * ns, cudaMemcpyDeviceToHost, st));
     const int m = (j + 1) * p;
     const bool check = (j + 1 >= next_check) || j + 1 == P.mb;
-    LAPY_CUDA_TRY(cudaStreamSynchronize(st));
     bool any_fail = false;
-    for (int s = 0; s < ns; ++s) any_fail |= (hact[s] && hfail[s]);
+    if (def.taken) {
+      StepStatus hs;
+      step_status_kernel<<<1, 256, 0, st>>>(ns * p, def.state, def.ctl, ns, e.fail, e.active, dstat);
+      LAPY_TRY(lapy_check_launch("step_status_kernel"));
+      LAPY_CUDA_TRY(cudaMemcpyAsync(&hs, dstat, sizeof(hs), cudaMemcpyDeviceToHost, st));
+      LAPY_CUDA_TRY(cudaStreamSynchronize(st));
+      LAPY_TRY(inner_done(hs.status, hs.iters));
+      any_fail = hs.fail != 0;
+    } else {
+      LAPY_CUDA_TRY(cudaMemcpyAsync(hfail.data(), e.fail, 4 * ns, cudaMemcpyDeviceToHost, st));
+      LAPY_CUDA_TRY(cudaStreamSynchronize(st));
+      for (int s = 0; s < ns; ++s) any_fail |= (hact[s] && hfail[s]);
+    }
     if (check || any_fail) {
       for (int s = 0; s < ns; ++s) hnsize[s] = m;
       LAPY_CUDA_TRY(cudaMemcpyAsync(e.nsize, hnsize.data(), 4 * ns, cudaMemcpyHostToDevice, st));
@@ -1338,20 +1397,22 @@ static int eigs_run(const EigPlan& P, const EigPtrs& e, const int32_t* indptr, c
       LAPY_CUDA_TRY(cudaMemcpyAsync(hnconv.data(), e.nconv, 4 * ns, cudaMemcpyDeviceToHost, st));
       LAPY_CUDA_TRY(cudaStreamSynchronize(st));
       all_done = true;
-      int missing = 0;
+      int64_t missing = 0;
       for (int s = 0; s < ns; ++s) {
         if (hact[s] && !hact2[s]) { res->status[s] = LAPY_OK; res->nbasis[s] = m; }
-        if (hact2[s]) missing = std::max(missing, k - hnconv[s]);
+        if (hact2[s]) missing += k - hnconv[s];
         hact[s] = hact2[s];
         all_done &= !hact[s];
       }
       int nact = 0;
       for (int s = 0; s < ns; ++s) nact += hact[s] != 0;
-      const double mm = (double)(m + p);
-      const double check_cost = kCheckSecPerCube * mm * mm * mm * (double)((nact + sms - 1) / sms);
-      const double step_cost = kStepSec + (double)step_pcg_iters * (kIterSec + kIterSecPerRow * (double)n);
+      const double check_cost = kCheckSecPerDim * (double)(m + p) * (1.0 + (double)nact / kCheckMeshes);
+      const double it = (double)step_pcg_iters;
+      const double step_cost = def.taken ? kChipStepSec + it * (kChipIterSec + kChipIterSecPerRow * (double)n)
+                                         : kGridStepSec + it * (kGridIterSec + kGridIterSecPerRow * (double)n);
       const int balanced = (int)std::lround(std::sqrt(2.0 * check_cost / step_cost));
-      next_check = j + 1 + std::max({1, (int)std::ceil(0.5 * missing / p), balanced});
+      const int steps = (int)std::lround((double)missing / std::max(1, nact) / (kPairsPerVector * p));
+      next_check = j + 1 + std::max({1, steps, balanced});
     }
   }
   res->blocks = j;

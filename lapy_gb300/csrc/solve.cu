@@ -53,17 +53,17 @@ static int residual64(const SysMatrix& K, const ChunkTable& ct, int p, const dou
 
 // The whole refined solve on chip (pcg_cluster.cu); rn2, st and ctl are
 // ir_solve's workspace.
-static int ir_solve_cluster(const SysMatrix& K, int nsp, int p, const double* B, double* X, double rtol,
-                            int maxiter, double inner_rtol, int max_rounds, double* rn2, int32_t* st, void* ctl,
-                            cudaStream_t stream, IrStats* stats, double* relres2_host, int32_t* state_host) {
-  PcgPrecondDesc<float> pc = K.pc32;
+// Launches of the on-chip solve; no wait.
+static int ir_launch_cluster(const SysMatrix& K, int nsp, int p, const double* B, double* X, double rtol, int maxiter,
+                             double inner_rtol, int max_rounds, double* rn2, int32_t* st, unsigned long long* ctl,
+                             cudaStream_t stream) {
   ClusterSolve c;
   c.n = K.n;
   c.indptr = K.indptr;
   c.indices = K.indices;
   c.k64 = K.k64;
   c.dinv = K.dinv32;
-  c.pc = &pc;
+  c.pc = &K.pc32;
   c.B = B;
   c.X = X;
   c.rtol = rtol;
@@ -72,11 +72,37 @@ static int ir_solve_cluster(const SysMatrix& K, int nsp, int p, const double* B,
   c.maxiter = maxiter;
   c.state = st;
   c.relres2 = rn2;
-  c.ctl = (unsigned long long*)(((uintptr_t)ctl + 255) & ~uintptr_t(255));
+  c.ctl = ctl;
   LAPY_CUDA_TRY(cudaMemsetAsync(c.ctl, 0, 64, stream));
   // segments without rows have no cluster: they are reported as solved
   LAPY_CUDA_TRY(cudaMemsetAsync(st, 0, sizeof(int32_t) * nsp, stream));
   LAPY_CUDA_TRY(cudaMemsetAsync(rn2, 0, sizeof(double) * nsp, stream));
+  return cluster_solve(*K.cluster, c, stream);
+}
+
+static bool takes_cluster(const SysMatrix& K, int p) {
+  return K.cluster && K.cluster->ok && K.cluster->p == p && !K.reliable &&
+         (K.pc32.kind == kPrecJacobi || K.pc32.kind == kPrecTwoLevel);
+}
+
+int ir_solve_deferred(const SysMatrix& K, const ChunkTable& ct, int p, const double* B, double* X, double rtol,
+                      int maxiter, double inner_rtol, int max_rounds, void* ws, size_t ws_bytes, cudaStream_t stream,
+                      IrDeferred* d) {
+  const int nsp = ct.nseg * p;
+  d->taken = takes_cluster(K, p) && !lapy_profile_enabled();
+  if (!d->taken) return LAPY_OK;
+  if (ws_bytes < ir_workspace_bytes(K.n, p, ct, 1, K.pc32.kind, K.pc32.nagg)) return LAPY_ERR_WORKSPACE;
+  char* w = (char*)(((uintptr_t)ws + 255) & ~uintptr_t(255));
+  double* rn2 = (double*)w; w += a256(sizeof(double) * nsp);
+  d->state = (int32_t*)w; w += a256(sizeof(int32_t) * nsp);
+  d->ctl = (unsigned long long*)w;
+  return ir_launch_cluster(K, nsp, p, B, X, rtol, maxiter, inner_rtol, max_rounds, rn2, d->state, d->ctl, stream);
+}
+
+static int ir_solve_cluster(const SysMatrix& K, int nsp, int p, const double* B, double* X, double rtol,
+                            int maxiter, double inner_rtol, int max_rounds, double* rn2, int32_t* st, void* ctl,
+                            cudaStream_t stream, IrStats* stats, double* relres2_host, int32_t* state_host) {
+  unsigned long long* dctl = (unsigned long long*)(((uintptr_t)ctl + 255) & ~uintptr_t(255));
   const bool prof = lapy_profile_enabled();
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (prof) {
@@ -84,14 +110,14 @@ static int ir_solve_cluster(const SysMatrix& K, int nsp, int p, const double* B,
     LAPY_CUDA_TRY(cudaEventCreate(&e1));
     LAPY_CUDA_TRY(cudaEventRecord(e0, stream));
   }
-  LAPY_TRY(cluster_solve(*K.cluster, c, stream));
+  LAPY_TRY(ir_launch_cluster(K, nsp, p, B, X, rtol, maxiter, inner_rtol, max_rounds, rn2, st, dctl, stream));
   if (prof) LAPY_CUDA_TRY(cudaEventRecord(e1, stream));
   std::vector<int32_t> hst(nsp);
   unsigned long long hctl[8];
   LAPY_CUDA_TRY(cudaMemcpyAsync(hst.data(), st, sizeof(int32_t) * nsp, cudaMemcpyDeviceToHost, stream));
   if (relres2_host)
     LAPY_CUDA_TRY(cudaMemcpyAsync(relres2_host, rn2, sizeof(double) * nsp, cudaMemcpyDeviceToHost, stream));
-  LAPY_CUDA_TRY(cudaMemcpyAsync(hctl, c.ctl, sizeof(hctl), cudaMemcpyDeviceToHost, stream));
+  LAPY_CUDA_TRY(cudaMemcpyAsync(hctl, dctl, sizeof(hctl), cudaMemcpyDeviceToHost, stream));
   LAPY_CUDA_TRY(cudaStreamSynchronize(stream));
   if (prof) {
     float ms = 0.f;
@@ -99,7 +125,7 @@ static int ir_solve_cluster(const SysMatrix& K, int nsp, int p, const double* B,
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     lapy_profile_add_pcg(ms, (long long)hctl[0], (long long)hctl[2], (long long)hctl[3], K.cluster->np,
-                         (int)sizeof(float), pc.kind, (double)hctl[4], true);
+                         (int)sizeof(float), K.pc32.kind, (double)hctl[4], true);
   }
   IrStats local;
   local.rounds = (int)hctl[1];
@@ -134,8 +160,7 @@ int ir_solve(const SysMatrix& K, const ChunkTable& ct, int p, const double* B, d
   const size_t pws_bytes = ws_bytes - (size_t)(w - (char*)ws);
   const int G = spmm_pick_group(n, K.nnz);
 
-  if (mixed && K.cluster && K.cluster->ok && K.cluster->p == p && !K.reliable &&
-      (precond == kPrecJacobi || precond == kPrecTwoLevel))
+  if (mixed && takes_cluster(K, p))
     return ir_solve_cluster(K, nsp, p, B, X, rtol, maxiter, inner_rtol, max_rounds, rn2, st, pws, stream, stats,
                             relres2_host, state_host);
 

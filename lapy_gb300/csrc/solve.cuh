@@ -42,6 +42,19 @@ int ir_solve(const SysMatrix& K, const ChunkTable& ct, int p, const double* B, d
              size_t ws_bytes, cudaStream_t stream, IrStats* stats, double* relres2_host,
              int32_t* state_host);
 
+// The same mixed solve launched without a wait, where the on-chip path takes it
+// (else `taken` is false and nothing was launched): state[s*p + c] and the
+// counters ctl (ctl[0]: PCG iterations) stay on the device, in the workspace,
+// until the next solve.
+struct IrDeferred {
+  bool taken = false;
+  int32_t* state = nullptr;
+  unsigned long long* ctl = nullptr;
+};
+int ir_solve_deferred(const SysMatrix& K, const ChunkTable& ct, int p, const double* B, double* X, double rtol,
+                      int maxiter, double inner_rtol, int max_rounds, void* ws, size_t ws_bytes, cudaStream_t stream,
+                      IrDeferred* d);
+
 // out = a*x + b*y on nnz values; y may be null.
 int vec_axpby(int64_t nnz, double a, const double* x, double b, const double* y, double* out,
               cudaStream_t stream);
