@@ -1398,9 +1398,15 @@ static int eigs_run(const EigPlan& P, const EigPtrs& e, const int32_t* indptr, c
       LAPY_CUDA_TRY(cudaStreamSynchronize(st));
       all_done = true;
       int64_t missing = 0;
+      int worst = 0;
+      int64_t rows_min = INT64_MAX;
       for (int s = 0; s < ns; ++s) {
         if (hact[s] && !hact2[s]) { res->status[s] = LAPY_OK; res->nbasis[s] = m; }
-        if (hact2[s]) missing += k - hnconv[s];
+        if (hact2[s]) {
+          missing += k - hnconv[s];
+          worst = std::max(worst, k - hnconv[s]);
+          rows_min = std::min<int64_t>(rows_min, P.ct.h_seg_row[s + 1] - P.ct.h_seg_row[s]);
+        }
         hact[s] = hact2[s];
         all_done &= !hact[s];
       }
@@ -1412,7 +1418,16 @@ static int eigs_run(const EigPlan& P, const EigPtrs& e, const int32_t* indptr, c
                                          : kGridStepSec + it * (kGridIterSec + kGridIterSecPerRow * (double)n);
       const int balanced = (int)std::lround(std::sqrt(2.0 * check_cost / step_cost));
       const int steps = (int)std::lround((double)missing / std::max(1, nact) / (kPairsPerVector * p));
-      next_check = j + 1 + std::max({1, steps, balanced});
+      int stride = std::max({1, steps, balanced});
+      // a basis that nears the rows of a mesh: short strides, and a check no
+      // later than the last block that fits (what a block adds beyond that is
+      // rounding noise, which Cholesky does not always flag)
+      if (rows_min < 2 * (int64_t)(j + 1 + stride) * p) {
+        stride = std::max(1, (worst + 2 * p - 1) / (2 * p));
+        const int64_t fits = rows_min / p;
+        if (fits > j + 1) stride = (int)std::min<int64_t>(stride, fits - (j + 1));
+      }
+      next_check = j + 1 + stride;
     }
   }
   res->blocks = j;
