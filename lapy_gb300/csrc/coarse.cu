@@ -6,8 +6,8 @@
 // in index order, neighbours in CSR order; segments are independent and run
 // on a fixed set of host threads).  Device: the Galerkin matrix W'KW of every
 // segment (one thread per coarse row, fixed summation order) and its dense
-// inverse (one CTA per segment: FP64 Cholesky, triangular inverse, B'B),
-// split into its dominant rank-1 term (FP32) and a BF16 remainder for the
+// inverse (FP64; up to kSweepMin aggregates one CTA per segment: Cholesky,
+// triangular inverse, B'B, above that block sweeps over the whole GPU), split into its dominant rank-1 term (FP32) and a BF16 remainder for the
 // per-iteration coarse product of the PCG.
 #include <algorithm>
 #include <atomic>

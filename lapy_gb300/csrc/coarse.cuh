@@ -23,7 +23,7 @@ size_t two_level_bytes(int64_t n, const int32_t* seg_row, int nseg, int nvc);
 
 // Build the coarse space of K (CSR on the device, FP64 values) for the
 // segments seg_row (host): aggregation on the host, Galerkin matrix W'KW and
-// its dense inverse (FP64 Cholesky, stored FP32) on the device, and the
+// its dense inverse (FP64; stored as a BF16 remainder and an FP32 mode) on the device, and the
 // split of the coarse work over the nvc virtual CTAs of the PCG's warp plan.
 // Fills the two-level fields of `pc` (which keeps its Jacobi diagonal).
 // `lab_in` (host, may be null): aggregate labels already planned

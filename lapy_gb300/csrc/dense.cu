@@ -1,5 +1,6 @@
 // Batched symmetric eigensolver for the small projected matrices of the
-// Lanczos iteration, FP64 throughout, one CTA per matrix:
+// Lanczos iteration, up to 384 rows one thread-block cluster per matrix
+// (sym_eig_cluster_kernel), above that one CTA:
 //   1. Householder reduction to tridiagonal form (Golub & Van Loan, Alg. 8.3.1),
 //   2. multisection on Sturm sequence counts for the wanted eigenvalues
 //      (Barth, Martin & Wilkinson 1967), several lanes per eigenvalue, with a
