@@ -9,11 +9,16 @@
 // search direction and the preconditioned residual in shared memory, where
 // neighbouring rows are read, through distributed shared memory when another
 // CTA of the cluster owns them; the FP32 matrix with 16-bit column codes in
-// shared memory.  An iteration is the Chronopoulos-Gear form of CG (w = K z,
-// q = w + beta q), so that both scalar products are one reduction: three
-// cluster barriers per iteration with the two-level preconditioner, two with
-// Jacobi.  Every CTA adds the partial sums of all CTAs in rank order, so each
-// takes the same decisions and a solve is reproducible to the bit.
+// shared memory.  Copies of neighbouring rows' directions are updated where
+// they are read (p = z + beta p; their owners store z), so that r'z is reduced
+// by the barrier that publishes z and q = K p, p'q are computed as plain CG
+// has them: three cluster barriers per iteration with the two-level
+// preconditioner, two with Jacobi.  (The Chronopoulos-Gear form, q by recurrence
+// and p'q = z'K z - beta r'z / alpha_old, needs no more barriers either, but the
+// difference cancels where K is close to singular in FP32: spheres of radius
+// 0.02 and 0.03 at sigma = -0.01 took up to 25 times the iterations or failed.)
+// Every CTA adds the partial sums of all CTAs in rank order, so each takes the
+// same decisions and a solve is reproducible to the bit.
 //
 // The FP64 refinement (true residual B - K X in FP64, FP32 correction solves)
 // runs in the same kernel: a solve is one launch per cluster size.
@@ -72,7 +77,7 @@ struct ClArgs {
   unsigned long long* ctl;
   int mat_smem, coarse_smem;
   // shared memory layout (byte offsets, the same in every CTA of a launch) and
-  // rows reserved for z (with its halo) and p
+  // rows reserved for the halo's z and for p (own rows and halo)
   int o_z, o_p, o_rc, o_yc, o_up, o_wp, o_mail, o_tab, o_push, o_val, o_code, o_coarse;
   int zrows, prows;
 };
@@ -233,12 +238,13 @@ __device__ __forceinline__ void cl_coarse(const uint16_t* kseg, int nc, int nrow
 // 32-row units a warp holds.  A CTA keeps its rows in slots of 32 per unit
 // (lanes past a unit's last row hold zero residuals and matrix entries, so the
 // iteration needs no masks), followed by the halo: copies of the neighbouring
-// rows of other CTAs, which their owners store after every update of z.
+// rows of other CTAs, whose z their owners store after every preconditioning.
 template <int NP, int UPW, bool TL>
 __global__ void __launch_bounds__(32 * kClMaxWarps, 1) ir_cluster_kernel(const ClArgs a, int cta_base) {
   extern __shared__ __align__(16) unsigned char sm[];
-  __shared__ float s_alpha[NP], s_beta[NP], s_vrc[NP];
-  __shared__ int s_done, s_rdone, s_mask;
+  __shared__ float s_vrc[NP];
+  __shared__ double s_rtol;
+  __shared__ int s_act, s_rdone, s_mask;
   const ClusterCta c = a.cta[cta_base + blockIdx.x];
   const unsigned rank = cl_rank(), cs = cl_size();
   const int lcs = 31 - __clz((int)cs);  // (a power of two)
@@ -248,17 +254,21 @@ __global__ void __launch_bounds__(32 * kClMaxWarps, 1) ir_cluster_kernel(const C
   const bool boss = warp == nwarp - 1;  // the warp that keeps the columns' scalars
   const int u0 = nunit * warp / nwarp, nu = nunit * (warp + 1) / nwarp - u0;
   const int slot0 = 32 * u0 + lane;  // slot of unit i of this warp: slot0 + 32 i
-  float* Z = reinterpret_cast<float*>(sm + a.o_z);
+  float* Z = reinterpret_cast<float*>(sm + a.o_z);  // halo rows only
   float* P = reinterpret_cast<float*>(sm + a.o_p);
   float* rc = reinterpret_cast<float*>(sm + a.o_rc);
   float* yc = reinterpret_cast<float*>(sm + a.o_yc);
   float* up = reinterpret_cast<float*>(sm + a.o_up);
-  float* wp = reinterpret_cast<float*>(sm + a.o_wp);  // per-warp partial sums (doubles in the residual stage)
-  // partial sums of every CTA, an area for each of the three reductions: an
-  // area is written again only after another cluster barrier
+  // per-warp partial sums and, from every CTA, their sums over its warps: an
+  // area for each of the three reductions (restriction, r'z, p'q), written again
+  // only after another barrier (the first: doubles in the residual stage)
+  float* wp = reinterpret_cast<float*>(sm + a.o_wp);
+  float* wp2 = wp + 16 * 2 * NP;
+  float* wp3 = wp2 + 16 * 2 * NP;
   float* mail = reinterpret_cast<float*>(sm + a.o_mail);
   float* mail2 = mail + 16 * 2 * NP;
-  double* mail64 = reinterpret_cast<double*>(mail2 + 16 * 3 * NP);
+  float* mail3 = mail2 + 16 * 2 * NP;
+  double* mail64 = reinterpret_cast<double*>(mail3 + 16 * NP);
   int32_t* ubase = reinterpret_cast<int32_t*>(sm + a.o_tab);   // slice start of every unit, relative
   int32_t* urow = ubase + nunit + 1;                           // first row, relative
   int32_t* uagg = urow + nunit + 1;                            // aggregate, relative to the CTA (0: none, with kv = 0)
@@ -297,8 +307,8 @@ __global__ void __launch_bounds__(32 * kClMaxWarps, 1) ir_cluster_kernel(const C
       aunit[g] = (ua - c.unit0) | ((ub - ua) << 16);
     }
   for (int i = threadIdx.x; i < h1 - h0; i += blockDim.x) push[i] = a.push[h0 + i];
-  for (int i = threadIdx.x; i < 16 * 4 * NP; i += blockDim.x) wp[i] = 0.f;
-  for (int i = threadIdx.x; i < 16 * 7 * NP; i += blockDim.x) mail[i] = 0.f;  // all three areas
+  for (int i = threadIdx.x; i < 16 * 5 * NP; i += blockDim.x) wp[i] = 0.f;    // all three areas
+  for (int i = threadIdx.x; i < 16 * 7 * NP; i += blockDim.x) mail[i] = 0.f;  // all four areas
   const float* val = a.val + e0;
   const uint16_t* code = a.code + e0;
   if (a.mat_smem) {
@@ -320,30 +330,29 @@ __global__ void __launch_bounds__(32 * kClMaxWarps, 1) ir_cluster_kernel(const C
   }
   __syncthreads();
 
-  float R[UPW][NP], Q[UPW][NP], X[UPW][NP], dv[UPW], dg[UPW];
+  float R[UPW][NP], X[UPW][NP], dv[UPW], dg[UPW];
   // global row of unit i of this warp and lane, or -1 past the unit's last row
   auto row_of = [&](int i) -> int64_t {
     if (i >= nu) return -1;
     const int r0 = urow[u0 + i];
     return lane < urow[u0 + i + 1] - r0 ? (int64_t)c.row0 + r0 + lane : -1;
   };
-  // NV per-warp values of `wp` summed over the CTA's warps and stored in every
+  // NV per-warp values of `part` summed over the CTA's warps and stored in every
   // CTA's area `area`; the caller passes a cluster barrier before it sums them
-  // with total() (one CTA: total() reads wp itself)
-  auto exchange = [&](float* area, int nv, int stride) {
+  // with total() (one CTA: total() reads `part` itself)
+  auto exchange = [&](const float* part, float* area, int nv) {
     __syncthreads();
     if (cs == 1) return;
     // (destination-major: the lanes of a store go to one CTA)
     for (int e = threadIdx.x; e < nv * (int)cs; e += blockDim.x) {
       const int dst = e / nv, v = e % nv;
-      const float s = sum16(wp + v, stride);
+      const float s = sum16(part + v, nv);
       if (dst == (int)rank) area[rank * nv + v] = s;
       else cl_store(cl_map(smem_u32(area + rank * nv + v), dst), s);
     }
   };
-  auto total = [&](const float* area, int nv, int stride) -> float {
-    if (lane >= nv) return 0.f;
-    return cs == 1 ? sum16(wp + lane, stride) : sum16(area + lane, nv);
+  auto total = [&](const float* part, const float* area, int nv) -> float {
+    return lane >= nv ? 0.f : sum16((cs == 1 ? part : area) + lane, nv);
   };
   // column sums over the cluster in FP64, on lanes 0..NP-1 of the boss warp
   auto reduce64 = [&](double (&acc)[NP]) -> double {
@@ -401,20 +410,28 @@ __global__ void __launch_bounds__(32 * kClMaxWarps, 1) ir_cluster_kernel(const C
   int iters = 0, rounds = 0;
   for (int round = 0; round < a.max_rounds; ++round) {
     ++rounds;
-    const float rtol2 = (float)(round_rtol * round_rtol);  // the boss warp's copy counts
+    const float rtol2 = (float)(round_rtol * round_rtol);
     // ---- FP32 PCG from zero on R
 #pragma unroll
     for (int i = 0; i < UPW; ++i) {
       float zero[NP];
 #pragma unroll
-      for (int q = 0; q < NP; ++q) { Q[i][q] = 0.f; X[i][q] = 0.f; zero[q] = 0.f; }
+      for (int q = 0; q < NP; ++q) { X[i][q] = 0.f; zero[q] = 0.f; }
       if (i < nu) cl_save<NP>(P, pplane, slot0 + 32 * i, zero);
     }
+    for (int h = threadIdx.x; h < c.nhalo; h += blockDim.x) {
+      float zero[NP];
+#pragma unroll
+      for (int q = 0; q < NP; ++q) zero[q] = 0.f;
+      cl_save<NP>(P, pplane, 32 * nunit + h, zero);
+    }
     __syncthreads();
-    int32_t st = kClActive;                    // column `lane` (boss warp)
-    float bb = 0.f, rgold = 0.f, raold = 0.f;  // its ||r0||^2, reciprocals of the last r'z and step (0: none yet)
+    // of column `lane`: its state and ||r0||^2 (two-level: in the boss warp),
+    // and the last r'z (0: none yet), the same in every warp
+    int32_t st = kClActive;
+    float bb = 0.f, rzold = 0.f;
     int it = 0;
-    // convergence of column `lane` from its squared residual (boss warp)
+    // convergence of column `lane` from its squared residual
     auto judge = [&](float rr) {
       if (it == 0) {
         bb = rr;
@@ -454,7 +471,7 @@ __global__ void __launch_bounds__(32 * kClMaxWarps, 1) ir_cluster_kernel(const C
             else if (v >= UPW * NP && v < NS) wp[warp * 2 * NP + v - UPW * NP] = t;
           }
         }
-        exchange(mail, 2 * NP, 2 * NP);
+        exchange(wp, mail, 2 * NP);
         if (nc > 0) {
           // (a warp per destination CTA; one CTA: all warps share it)
           const int step = 32 * (nwarp >> lcs > 0 ? nwarp >> lcs : 1);
@@ -488,80 +505,134 @@ __global__ void __launch_bounds__(32 * kClMaxWarps, 1) ir_cluster_kernel(const C
         }
         cl_sync(cs);
         if (boss) {
-          const float s = total(mail, 2 * NP, 2 * NP);
+          const float s = total(wp, mail, 2 * NP);
           if (lane >= NP && lane < 2 * NP) s_vrc[lane - NP] = cscale * s;
           if (lane < NP) judge(s);
-          const bool any = __any_sync(0xffffffffu, lane < NP && st == kClActive);
-          if (lane == 0) s_done = !any || it >= a.maxiter;
+          const unsigned m = __ballot_sync(0xffffffffu, lane < NP && st == kClActive);
+          if (lane == 0) s_act = it < a.maxiter ? (int)m : 0;
         }
         if (nc > 0) {  // (two calls, so that the compiler knows the address space)
           if (a.coarse_smem) cl_coarse<NP>(reinterpret_cast<const uint16_t*>(sm + a.o_coarse), nc, nagg, rc, yc);
           else cl_coarse<NP>(kseg, nc, nagg, rc, yc);
         }
         __syncthreads();
-        if (s_done) break;
+        if (s_act == 0) break;
       }
       // ---- z = D^-1 r (+ the coarse correction), r'z (and ||r||^2 for Jacobi)
-      constexpr int NV = TL ? 2 * NP : 4 * NP;  // partial sums per warp: r'z, z'w (, ||r||^2)
-      float red[NV];
-#pragma unroll
-      for (int v = 0; v < NV; ++v) red[v] = 0.f;
+      constexpr int NV = TL ? NP : 2 * NP;  // partial sums per warp
+      float z[UPW][NP];
       {
+        float red[NV];
+#pragma unroll
+        for (int v = 0; v < NV; ++v) red[v] = 0.f;
 #pragma unroll
         for (int i = 0; i < UPW; ++i) {
           if (i < nu) {
-            float z[NP];
 #pragma unroll
-            for (int q = 0; q < NP; ++q) z[q] = dv[i] * R[i][q];
+            for (int q = 0; q < NP; ++q) z[i][q] = dv[i] * R[i][q];
             if constexpr (TL) {
               const float* y = yc + uagg[u0 + i] * NP;
               const float kv = ukv[u0 + i];
 #pragma unroll
-              for (int q = 0; q < NP; ++q) z[q] += y[q] + kv * s_vrc[q];
+              for (int q = 0; q < NP; ++q) z[i][q] += y[q] + kv * s_vrc[q];
             }
-            cl_save<NP>(Z, zplane, slot0 + 32 * i, z);
 #pragma unroll
             for (int q = 0; q < NP; ++q) {
-              red[q] = fmaf(R[i][q], z[q], red[q]);
-              if constexpr (!TL) red[2 * NP + q] = fmaf(R[i][q], R[i][q], red[2 * NP + q]);
+              red[q] = fmaf(R[i][q], z[i][q], red[q]);
+              if constexpr (!TL) red[NP + q] = fmaf(R[i][q], R[i][q], red[NP + q]);
             }
           }
         }
-        if (cs > 1) {  // copies for the neighbours (this warp's rows)
-          __syncwarp();
-          for (int e = upush[u0] + lane; e < upush[u0 + nu]; e += 32) {
-            const unsigned w = push[e];  // slot (12 bits), rank (4), halo slot (16)
-            const int src = (int)(w & 4095u);
-            const unsigned dst = w >> 16, rk = (w >> 12) & 15u;
-            float x[NP];
-            cl_load<NP>(Z, zplane, src, x);
-            const unsigned ra = cl_map(smem_u32(Z), rk);
-            if constexpr (NP >= 4) {
+        constexpr int per = 32 / NV;
+        const float t = lane_totals<NV>(red);
+        if (lane % per == 0) wp2[warp * NV + lane / per] = t;
+      }
+      if (cs > 1) {  // copies for the neighbours (this warp's rows)
 #pragma unroll
-              for (int h = 0; h < NP / 4; ++h)
-                cl_store4(ra + 4u * (unsigned)(h * zplane) + 16u * dst, x[4 * h], x[4 * h + 1], x[4 * h + 2], x[4 * h + 3]);
-            } else if constexpr (NP == 2) {
-              cl_store2(ra + 8u * dst, x[0], x[1]);
-            } else {
-              cl_store(ra + 4u * dst, x[0]);
+        for (int i = 0; i < UPW; ++i) {
+          if (i < nu) {
+            const int e1 = upush[u0 + i + 1];
+            for (int e0 = upush[u0 + i]; e0 < e1; e0 += 32) {
+              const unsigned w = push[min(e0 + lane, e1 - 1)];  // slot (12 bits), rank (4), halo row (16)
+              const unsigned dst = w >> 16, rk = (w >> 12) & 15u;
+              float x[NP];
+#pragma unroll
+              for (int q = 0; q < NP; ++q) x[q] = __shfl_sync(0xffffffffu, z[i][q], (int)(w & 31u));
+              if (e0 + lane < e1) {
+                const unsigned ra = cl_map(smem_u32(Z), rk);
+                if constexpr (NP >= 4) {
+#pragma unroll
+                  for (int h = 0; h < NP / 4; ++h)
+                    cl_store4(ra + 4u * (unsigned)(h * zplane) + 16u * dst, x[4 * h], x[4 * h + 1], x[4 * h + 2],
+                              x[4 * h + 3]);
+                } else if constexpr (NP == 2) {
+                  cl_store2(ra + 8u * dst, x[0], x[1]);
+                } else {
+                  cl_store(ra + 4u * dst, x[0]);
+                }
+              }
             }
           }
         }
       }
-      cl_sync(cs);
-      // ---- w = K z, z'w
-      float W[UPW][NP];
+      exchange(wp2, mail2, NV);
+      if (cs > 1) cl_sync(cs);
+      // ---- beta, p = z + beta p in the CTA's rows and its copies (scalars of
+      // column `lane` in every warp)
+      float gam = total(wp2, mail2, NV);
+      bool act;
+      if constexpr (TL) {
+        act = (s_act >> lane) & 1;
+      } else {
+        const float rr = __shfl_sync(0xffffffffu, gam, (lane + NP) & 31);
+        if (lane < NP) judge(rr);
+        act = lane < NP && st == kClActive && it < a.maxiter;
+        if (!__any_sync(0xffffffffu, act)) break;
+      }
+      if (act && !(gam > 0.f && isfinite(gam))) {
+        st = isfinite(gam) ? LAPY_ERR_BREAKDOWN : LAPY_ERR_NAN;
+        act = false;
+      }
       {
+        const float b = act && rzold > 0.f ? gam / rzold : 0.f;
+        rzold = gam;
+        float be[NP];
+#pragma unroll
+        for (int q = 0; q < NP; ++q) be[q] = __shfl_sync(0xffffffffu, b, q);
+#pragma unroll
+        for (int i = 0; i < UPW; ++i) {
+          if (i < nu) {
+            float pv[NP];
+            cl_load<NP>(P, pplane, slot0 + 32 * i, pv);
+#pragma unroll
+            for (int q = 0; q < NP; ++q) pv[q] = fmaf(be[q], pv[q], z[i][q]);
+            cl_save<NP>(P, pplane, slot0 + 32 * i, pv);
+          }
+        }
+        for (int h = threadIdx.x; h < c.nhalo; h += blockDim.x) {
+          float zv[NP], pv[NP];
+          cl_load<NP>(Z, zplane, h, zv);
+          cl_load<NP>(P, pplane, 32 * nunit + h, pv);
+#pragma unroll
+          for (int q = 0; q < NP; ++q) pv[q] = fmaf(be[q], pv[q], zv[q]);
+          cl_save<NP>(P, pplane, 32 * nunit + h, pv);
+        }
+      }
+      __syncthreads();
+      // ---- q = K p, p'q
+      float Q[UPW][NP];
+      {
+        float red[NP];
+#pragma unroll
+        for (int q = 0; q < NP; ++q) red[q] = 0.f;
 #pragma unroll
         for (int i = 0; i < UPW; ++i) {
 #pragma unroll
-          for (int q = 0; q < NP; ++q) W[i][q] = 0.f;
+          for (int q = 0; q < NP; ++q) Q[i][q] = 0.f;
           if (i < nu) {
             const int b0 = ubase[u0 + i], b1 = ubase[u0 + i + 1];
             const float2* vp = reinterpret_cast<const float2*>(val + b0) + lane;
             const uint32_t* cp = reinterpret_cast<const uint32_t*>(code + b0) + lane;
-            float z[NP];
-            cl_load<NP>(Z, zplane, slot0 + 32 * i, z);
             // pairs of entries of the lane's row, two pairs at a time
             int k = (b1 - b0) >> 6;
 #pragma unroll 1
@@ -569,99 +640,74 @@ __global__ void __launch_bounds__(32 * kClMaxWarps, 1) ir_cluster_kernel(const C
               const uint32_t ca = cp[0], cb = cp[32];
               const float2 va = vp[0], vb = vp[32];
               float x0[NP], x1[NP], x2[NP], x3[NP];
-              cl_load<NP>(Z, zplane, ca & 0xffff, x0);
-              cl_load<NP>(Z, zplane, ca >> 16, x1);
-              cl_load<NP>(Z, zplane, cb & 0xffff, x2);
-              cl_load<NP>(Z, zplane, cb >> 16, x3);
+              cl_load<NP>(P, pplane, ca & 0xffff, x0);
+              cl_load<NP>(P, pplane, ca >> 16, x1);
+              cl_load<NP>(P, pplane, cb & 0xffff, x2);
+              cl_load<NP>(P, pplane, cb >> 16, x3);
 #pragma unroll
               for (int q = 0; q < NP; ++q) {
-                W[i][q] = fmaf(va.x, x0[q], W[i][q]);
-                W[i][q] = fmaf(va.y, x1[q], W[i][q]);
-                W[i][q] = fmaf(vb.x, x2[q], W[i][q]);
-                W[i][q] = fmaf(vb.y, x3[q], W[i][q]);
+                Q[i][q] = fmaf(va.x, x0[q], Q[i][q]);
+                Q[i][q] = fmaf(va.y, x1[q], Q[i][q]);
+                Q[i][q] = fmaf(vb.x, x2[q], Q[i][q]);
+                Q[i][q] = fmaf(vb.y, x3[q], Q[i][q]);
               }
             }
             if (k) {
               const uint32_t ca = cp[0];
               const float2 va = vp[0];
               float x0[NP], x1[NP];
-              cl_load<NP>(Z, zplane, ca & 0xffff, x0);
-              cl_load<NP>(Z, zplane, ca >> 16, x1);
+              cl_load<NP>(P, pplane, ca & 0xffff, x0);
+              cl_load<NP>(P, pplane, ca >> 16, x1);
 #pragma unroll
               for (int q = 0; q < NP; ++q) {
-                W[i][q] = fmaf(va.x, x0[q], W[i][q]);
-                W[i][q] = fmaf(va.y, x1[q], W[i][q]);
+                Q[i][q] = fmaf(va.x, x0[q], Q[i][q]);
+                Q[i][q] = fmaf(va.y, x1[q], Q[i][q]);
               }
             }
+            float pv[NP];
+            cl_load<NP>(P, pplane, slot0 + 32 * i, pv);
 #pragma unroll
             for (int q = 0; q < NP; ++q) {
-              W[i][q] = fmaf(dg[i], z[q], W[i][q]);
-              red[NP + q] = fmaf(z[q], W[i][q], red[NP + q]);
+              Q[i][q] = fmaf(dg[i], pv[q], Q[i][q]);
+              red[q] = fmaf(pv[q], Q[i][q], red[q]);
             }
           }
         }
-        constexpr int per = 32 / NV;
-        const float t = lane_totals<NV>(red);
-        if (lane % per == 0) wp[warp * NV + lane / per] = t;
+        constexpr int per = 32 / NP;
+        const float t = lane_totals<NP>(red);
+        if (lane % per == 0) wp3[warp * NP + lane / per] = t;
       }
-      constexpr int NM = TL ? 2 * NP : 3 * NP;
-      exchange(mail2, NM, NV);
+      exchange(wp3, mail3, NP);
       if (cs > 1) cl_sync(cs);
-      if (boss) {
-        const float s = total(mail2, NM, NV);
-        const float del = __shfl_sync(0xffffffffu, s, (lane + NP) & 31);
-        if constexpr (!TL) {
-          const float rr = __shfl_sync(0xffffffffu, s, (lane + 2 * NP) & 31);
-          if (lane < NP) judge(rr);
-        }
-        float alpha = 0.f, beta = 0.f;
-        if (lane < NP && st == kClActive && it < a.maxiter) {
-          const float gam = s;
-          if (!isfinite(gam) || !isfinite(del)) st = LAPY_ERR_NAN;
-          else if (!(gam > 0.f) || !(del > 0.f)) st = LAPY_ERR_BREAKDOWN;
-          else {
-            // p'Kp = z'Kz - beta^2 p_old'K p_old; a direction whose estimate
-            // cancels away is dropped (steepest descent from here)
-            beta = gam * rgold;
-            float pq = del - beta * (gam * raold);
-            if (!(pq > 0.f)) { beta = 0.f; pq = del; }
+      // ---- x += alpha p, r -= alpha q
+      {
+        const float pq = total(wp3, mail3, NP);
+        float alpha = 0.f;
+        if (act) {
+          if (!(pq > 0.f) || !isfinite(pq)) {
+            st = LAPY_ERR_BREAKDOWN;
+          } else {
             alpha = gam / pq;
-            if (!isfinite(alpha)) { alpha = 0.f; beta = 0.f; st = LAPY_ERR_NAN; }
-            rgold = 1.f / gam;
-            raold = 1.f / alpha;
+            if (!isfinite(alpha)) {
+              alpha = 0.f;
+              st = LAPY_ERR_NAN;
+            }
           }
         }
-        if (lane < NP) {
-          s_alpha[lane] = alpha;
-          s_beta[lane] = beta;
-        }
-        if constexpr (!TL) {
-          const bool any = __any_sync(0xffffffffu, lane < NP && st == kClActive);
-          if (lane == 0) s_done = !any || it >= a.maxiter;
-        }
-      }
-      __syncthreads();
-      if constexpr (!TL) {
-        if (s_done) break;
-      }
-      // ---- p = z + beta p, q = w + beta q, x += alpha p, r -= alpha q
-      float al[NP], be[NP];
+        float al[NP];
 #pragma unroll
-      for (int q = 0; q < NP; ++q) { al[q] = s_alpha[q]; be[q] = s_beta[q]; }
+        for (int q = 0; q < NP; ++q) al[q] = __shfl_sync(0xffffffffu, alpha, q);
 #pragma unroll
-      for (int i = 0; i < UPW; ++i) {
-        if (i < nu) {
-          float z[NP], pv[NP];
-          cl_load<NP>(Z, zplane, slot0 + 32 * i, z);
-          cl_load<NP>(P, pplane, slot0 + 32 * i, pv);
+        for (int i = 0; i < UPW; ++i) {
+          if (i < nu) {
+            float pv[NP];
+            cl_load<NP>(P, pplane, slot0 + 32 * i, pv);
 #pragma unroll
-          for (int q = 0; q < NP; ++q) {
-            pv[q] = fmaf(be[q], pv[q], z[q]);
-            Q[i][q] = fmaf(be[q], Q[i][q], W[i][q]);
-            X[i][q] = fmaf(al[q], pv[q], X[i][q]);
-            R[i][q] = fmaf(-al[q], Q[i][q], R[i][q]);
+            for (int q = 0; q < NP; ++q) {
+              X[i][q] = fmaf(al[q], pv[q], X[i][q]);
+              R[i][q] = fmaf(-al[q], Q[i][q], R[i][q]);
+            }
           }
-          cl_save<NP>(P, pplane, slot0 + 32 * i, pv);
         }
       }
     }
@@ -727,15 +773,16 @@ __global__ void __launch_bounds__(32 * kClMaxWarps, 1) ir_cluster_kernel(const C
       double need = 1.0;
       if (lane < NP && !masked && hr > 0.0) need = fmin(1.0, 0.25 * a.rtol * sqrt(hb / hr));
       for (int o = 16; o > 0; o >>= 1) need = fmin(need, __shfl_xor_sync(0xffffffffu, need, o));
-      round_rtol = fmax(a.inner_rtol, fmin(0.5, need));
       const unsigned mk = __ballot_sync(0xffffffffu, lane >= NP || masked);
       if (lane == 0) {
+        s_rtol = fmax(a.inner_rtol, fmin(0.5, need));
         s_mask = (int)mk;
         s_rdone = mk == 0xffffffffu;
       }
     }
     __syncthreads();
     const int mk = s_mask;
+    round_rtol = s_rtol;
     if (s_rdone) break;
 #pragma unroll
     for (int i = 0; i < UPW; ++i)
@@ -843,15 +890,14 @@ __global__ void cl_halo_kernel(const ClSplitCta* __restrict__ split, const int32
 
 // Push lists of the owners (the order within a unit's list does not matter).
 __global__ void cl_push_kernel(const ClSplitCta* __restrict__ split, const int32_t* __restrict__ row_slot,
-                               const int32_t* __restrict__ cta_unit0, const int32_t* __restrict__ cta_units,
-                               const uint32_t* __restrict__ bits, const int32_t* __restrict__ rank,
+                               const int32_t* __restrict__ cta_unit0, const uint32_t* __restrict__ bits, const int32_t* __restrict__ rank,
                                const int32_t* __restrict__ push_ptr, int32_t* __restrict__ push_fill,
                                uint32_t* __restrict__ push) {
   const ClSplitCta c = split[blockIdx.x];
-  const int nw = (c.seg1 - c.seg0 + 31) >> 5, own = 32 * cta_units[blockIdx.x];
+  const int nw = (c.seg1 - c.seg0 + 31) >> 5;
   const uint32_t me = (uint32_t)(blockIdx.x - c.first);
   for (int i = threadIdx.x; i < nw; i += blockDim.x) {
-    int at = own + rank[c.word0 + i];
+    int at = rank[c.word0 + i];
     for (uint32_t m = bits[c.word0 + i]; m; m &= m - 1, ++at) {
       const int rs = row_slot[c.seg0 + 32 * i + __ffs(m) - 1];
       const int u = cta_unit0[rs >> 12] + ((rs & 4095) >> 5);
@@ -913,8 +959,8 @@ __global__ void cl_fill_kernel(int nunit, const int32_t* __restrict__ unit_row, 
 // ---- kernel variants -------------------------------------------------------------
 using ClKernel = void (*)(const ClArgs, int);
 
-// Units a warp holds, by columns: four NP-wide register rows per unit (r, q,
-// w, x), 48 registers at most, so that 16 warps fit without spilling.
+// Units a warp holds, by columns: three NP-wide register rows per unit (r, x,
+// and z or q), 36 registers at most, so that 16 warps fit without spilling.
 struct ClVariant {
   int np, upw;
   ClKernel tl, jacobi;
@@ -946,12 +992,12 @@ static size_t class_layout(const ClusterClass& k, int np, bool tl, bool mat, boo
     return (int)o;
   };
   const size_t row = 4 * (size_t)np;
-  const int zrows = k.slots, prows = 32 * k.units;
+  const int zrows = k.halo, prows = k.slots;
   const int oz = take(row * zrows), op = take(row * prows);
   const int orc = take(tl ? row * k.ld : 0), oyc = take(tl ? row * std::max(k.aggs, 1) : 0);
   const int oup = take(tl ? row * k.units : 0);
-  const int owp = take(16 * (size_t)np * 16);           // 4 NP floats (or NP doubles) per warp
-  const int omail = take(448 * (size_t)np);             // 16 CTAs x (2 NP + 3 NP floats, NP doubles)
+  const int owp = take(320 * (size_t)np);               // 16 warps x (2 NP + 2 NP + NP floats; NP doubles)
+  const int omail = take(448 * (size_t)np);             // 16 CTAs x (2 NP + 2 NP + NP floats, NP doubles)
   const int otab = take(4 * (5 * (size_t)k.units + 3 + (size_t)(tl ? k.aggs : 0)));
   const int opush = take(4 * (size_t)k.push);
   const int oval = take(mat ? 4 * (size_t)k.elems : 0), ocode = take(mat ? 2 * (size_t)k.elems : 0);
@@ -1228,6 +1274,8 @@ int cluster_plan(int64_t n, int64_t nnz, const int32_t* indptr, const int32_t* i
         c.seg = s;
         c.col0 = g * np;
         k.units = std::max(k.units, ub - ua);
+        c.nhalo = halo[q];
+        k.halo = std::max(k.halo, halo[q]);
         k.slots = std::max(k.slots, 32 * (ub - ua) + halo[q]);
         k.aggs = std::max(k.aggs, c.agg1 - c.agg0);
         k.push = std::max(k.push, pptr[ub] - pptr[ua]);
@@ -1259,7 +1307,7 @@ int cluster_plan(int64_t n, int64_t nnz, const int32_t* indptr, const int32_t* i
   LAPY_TRY(put(d_cta, cta.data(), sizeof(ClusterCta) * cta.size()));
   if (npush > 0) {
     LAPY_CUDA_TRY(cudaMemsetAsync(d_cnt, 0, 4 * (size_t)(nunit + 1), stream));
-    cl_push_kernel<<<nsplit, 256, 0, stream>>>(d_spl, d_slot, d_cu0, d_cun, d_bits, d_rank, d_pp, d_cnt, d_push);
+    cl_push_kernel<<<nsplit, 256, 0, stream>>>(d_spl, d_slot, d_cu0, d_bits, d_rank, d_pp, d_cnt, d_push);
     LAPY_TRY(lapy_check_launch("cl_push_kernel"));
   }
   cl_fill_kernel<<<blocks, 256, 0, stream>>>(nunit, d_row, d_uct, d_cu0, d_cun, d_spl, d_slot, d_bits, d_rank, indptr,

@@ -9,13 +9,14 @@
 
 namespace lapy {
 
-// One CTA of a cluster: its rows, its 32-row units, its aggregates (two-level)
-// and the first of the columns its cluster solves.
+// One CTA of a cluster: its rows, its 32-row units, its aggregates (two-level),
+// the first of the columns its cluster solves and its copies of other CTAs' rows.
 struct ClusterCta {
   int32_t row0, row1;
   int32_t unit0, unit1;
   int32_t agg0, agg1;
   int32_t seg, col0;
+  int32_t nhalo;
 };
 
 // Clusters of one size: a launch.
@@ -24,7 +25,7 @@ struct ClusterClass {
   int warps = 16;    // warps per CTA
   const void* kernel = nullptr;
   int cta0 = 0, ncta = 0;
-  int slots = 0, units = 0, aggs = 0, ld = 0, push = 0;  // largest of the class
+  int slots = 0, halo = 0, units = 0, aggs = 0, ld = 0, push = 0;  // largest of the class
   int64_t elems = 0;
   bool mat_smem = true;  // matrix in shared memory (else read through L2)
   bool coarse_smem = true;  // rows of the coarse inverse likewise
@@ -54,7 +55,7 @@ struct ClusterPlan {
   const float* val = nullptr;           // device
   const float* diag = nullptr;          // device, 32 nunit
   const int32_t* push_ptr = nullptr;    // device, nunit + 1: halo copies to store, per unit of the owner
-  const uint32_t* push = nullptr;       // device: slot | CTA of the cluster << 12 | halo slot there << 16
+  const uint32_t* push = nullptr;       // device: slot | CTA of the cluster << 12 | halo row there << 16
 };
 
 // Plan the clusters for p columns and build the packed FP32 matrix into
