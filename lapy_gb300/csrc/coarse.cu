@@ -936,6 +936,7 @@ int build_two_level(int64_t n, const int32_t* indptr, const int32_t* indices, co
   LAPY_CUDA_TRY(cudaMemcpyAsync(d_offp, off_pad.data(), 8 * off_pad.size(), cudaMemcpyHostToDevice, stream));
   if (off[nseg] > 0) LAPY_CUDA_TRY(cudaMemsetAsync(d_kc, 0, 8 * (size_t)off[nseg], stream));
   LAPY_CUDA_TRY(cudaMemsetAsync(d_fail, 0, 4 * (size_t)nseg, stream));
+  LAPY_CUDA_TRY(cudaMemsetAsync(d_kscale, 0, 4 * (size_t)nseg, stream));  // segments without aggregates keep the zero
   if (nagg > 0) {
     coarse_galerkin_kernel<<<lapy_ceil_div(nagg, 128), 128, 0, stream>>>(nagg, d_agg, d_ptr, d_row, d_sid, d_seg, d_off,
                                                                          indptr, indices, k64, d_kc);

@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(32 * kClMaxWarps, 1) ir_cluster_kernel(const C
     segbase = a.seg_agg[c.seg];
     nc = a.seg_agg[c.seg + 1] - segbase;
     ld = (nc + 7) & ~7;
-    cscale = a.kscale[c.seg];
+    cscale = nc > 0 ? a.kscale[c.seg] : 0.f;  // (a segment without aggregates has no coarse space)
     kseg = a.kinv + a.kinv_off[c.seg] + (int64_t)(c.agg0 - segbase) * ld;  // this CTA's rows of the coarse inverse
   }
 
