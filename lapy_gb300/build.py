@@ -53,7 +53,7 @@ def sources() -> list[Path]:
 
 def _compile(src: Path, nvcc: str) -> Path:
     obj = BUILD_DIR / (src.name + ".o")
-    deps = [src, *CSRC.glob("*.cuh"), *INCLUDE.glob("*.h")]
+    deps = [src, *CSRC.glob("*.cuh"), *CSRC.glob("*.h"), *INCLUDE.glob("*.h")]
     if obj.exists() and obj.stat().st_mtime >= max(d.stat().st_mtime for d in deps):
         return obj
     extra_env = os.environ.get("LAPY_NVCC_FLAGS", "").split()

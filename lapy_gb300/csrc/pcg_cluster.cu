@@ -35,6 +35,7 @@
 #include <cmath>
 #include <vector>
 #include "cluster.cuh"
+#include "fork_join.h"
 #include "pcg_cluster.cuh"
 #include "scan.cuh"
 
@@ -1363,9 +1364,10 @@ int cluster_solve(const ClusterPlan& plan, const ClusterSolve& s, cudaStream_t s
   a.state = s.state;
   a.relres2 = s.relres2;
   a.ctl = s.ctl;
-  const bool fork = plan.cls.size() > 1;
+  const int ncls = (int)plan.cls.size();
+  const bool fork = ncls > 1;
   if (fork) LAPY_CUDA_TRY(cudaEventRecord(plan.events.back(), stream));
-  for (size_t i = 0; i < plan.cls.size(); ++i) {
+  auto begin = [&](int i) -> int {
     const ClusterClass& k = plan.cls[i];
     cudaStream_t on = fork ? plan.streams[i] : stream;
     if (fork) LAPY_CUDA_TRY(cudaStreamWaitEvent(on, plan.events.back(), 0));
@@ -1376,12 +1378,19 @@ int cluster_solve(const ClusterPlan& plan, const ClusterSolve& s, cudaStream_t s
     cudaLaunchAttribute attr;
     launch_config(k, on, &cfg, &attr);
     LAPY_CUDA_TRY(cudaLaunchKernelEx(&cfg, (ClKernel)k.kernel, (const ClArgs)a, k.cta0));
-    LAPY_TRY(lapy_check_launch("ir_cluster_kernel"));
-    if (fork) LAPY_CUDA_TRY(cudaEventRecord(plan.events[i], on));
-  }
-  // (all forks before the first join: a launch that failed leaves none running unjoined)
-  for (size_t i = 0; fork && i < plan.cls.size(); ++i) LAPY_CUDA_TRY(cudaStreamWaitEvent(stream, plan.events[i], 0));
-  return LAPY_OK;
+    return lapy_check_launch("ir_cluster_kernel");
+  };
+  // the caller's stream waits for the class; where that fails, the host does
+  auto join = [&](int i) -> int {
+    if (!fork) return LAPY_OK;
+    if (cudaEventRecord(plan.events[i], plan.streams[i]) == cudaSuccess &&
+        cudaStreamWaitEvent(stream, plan.events[i], 0) == cudaSuccess)
+      return LAPY_OK;
+    cudaGetLastError();
+    LAPY_CUDA_TRY(cudaStreamSynchronize(plan.streams[i]));
+    return LAPY_OK;
+  };
+  return fork_join(ncls, begin, join);
 }
 
 }  // namespace lapy
