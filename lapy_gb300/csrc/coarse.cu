@@ -730,7 +730,7 @@ int plan_aggregate_order(int64_t n, const int32_t* hptr, const int32_t* hidx, co
 int build_two_level(int64_t n, const int32_t* indptr, const int32_t* indices, const double* k64,
                     const int32_t* seg_row, int nseg, int nvc, void* mem, size_t bytes,
                     PcgPrecondDesc<float>* pc, cudaStream_t stream, const int32_t* lab_in, int agg_target,
-                    std::vector<int32_t>* h_seg_agg, std::vector<int32_t>* h_agg_ptr) {
+                    std::vector<int32_t>* h_seg_agg, std::vector<int32_t>* h_agg_rows) {
   nvc = std::max(nvc, 1);
   if (bytes < two_level_bytes(n, seg_row, nseg, nvc)) return LAPY_ERR_WORKSPACE;
   std::vector<int32_t> lab(n, -1), nc(nseg, 0);
@@ -954,7 +954,16 @@ int build_two_level(int64_t n, const int32_t* indptr, const int32_t* indices, co
   // the host vectors are pageable: the copies complete before they go away
   LAPY_CUDA_TRY(cudaStreamSynchronize(stream));
   if (h_seg_agg) *h_seg_agg = seg_agg;
-  if (h_agg_ptr) *h_agg_ptr = agg_ptr;
+  if (h_agg_rows) {
+    h_agg_rows->clear();
+    if (contiguous) {
+      h_agg_rows->resize(2 * (size_t)nagg);
+      for (int g = 0; g < nagg; ++g) {
+        (*h_agg_rows)[2 * g] = agg_row[agg_ptr[g]];
+        (*h_agg_rows)[2 * g + 1] = agg_row[agg_ptr[g + 1] - 1] + 1;
+      }
+    }
+  }
   pc->kind = kPrecTwoLevel;
   pc->nagg = nagg;
   pc->agg = d_agg;
@@ -962,7 +971,9 @@ int build_two_level(int64_t n, const int32_t* indptr, const int32_t* indices, co
   pc->agg_row = d_row;
   pc->agg_sid = d_sid;
   pc->seg_agg = d_seg;
-  pc->agg_contig = contiguous ? 1 : 0;
+  // (agg_ptr counts the rows of aggregates only: it names rows where none lies
+  // before an aggregate without belonging to one, as in a segment with none)
+  pc->agg_contig = contiguous && (nagg == 0 || agg_row.back() + 1 == (int32_t)agg_row.size()) ? 1 : 0;
   pc->kinv_off = d_offp;
   pc->kinv = d_kinv;
   pc->kvec = d_kvec;

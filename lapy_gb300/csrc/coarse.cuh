@@ -27,13 +27,15 @@ size_t two_level_bytes(int64_t n, const int32_t* seg_row, int nseg, int nvc);
 // split of the coarse work over the nvc virtual CTAs of the PCG's warp plan.
 // Fills the two-level fields of `pc` (which keeps its Jacobi diagonal).
 // `lab_in` (host, may be null): aggregate labels already planned
-// (plan_aggregate_order), used instead of aggregating here.  h_seg_agg,
-// h_agg_ptr (may be null) receive the host copies of those tables.
+// (plan_aggregate_order), used instead of aggregating here.  h_seg_agg (may be
+// null) receives the host copy of the aggregates per segment, h_agg_rows (may
+// be null) the first row and the end of every aggregate, or nothing when the
+// rows of an aggregate do not lie side by side.
 int build_two_level(int64_t n, const int32_t* indptr, const int32_t* indices, const double* k64,
                     const int32_t* seg_row, int nseg, int nvc, void* mem, size_t bytes,
                     PcgPrecondDesc<float>* pc, cudaStream_t stream, const int32_t* lab_in = nullptr,
                     int agg_target = kAggTarget, std::vector<int32_t>* h_seg_agg = nullptr,
-                    std::vector<int32_t>* h_agg_ptr = nullptr);
+                    std::vector<int32_t>* h_agg_rows = nullptr);
 
 // Row order of a batch (host, pattern on the host) that makes every
 // aggregate a contiguous row range: each segment is aggregated as

@@ -1258,15 +1258,15 @@ static int eigs_run(const EigPlan& P, const EigPtrs& e, const int32_t* indptr, c
   K.k64 = e.k64; K.k32 = e.k32; K.dinv64 = e.dinv64; K.dinv32 = e.dinv32;
   // inner solves: on chip when every mesh fits, else the persistent PCG on
   // SELL copies of K
-  std::vector<int32_t> h_seg_agg, h_agg_ptr;
+  std::vector<int32_t> h_seg_agg, h_agg_rows;
   if (P.precond == kPrecTwoLevel)
     LAPY_TRY(build_two_level(n, indptr, indices, e.k64, P.ct.h_seg_row.data(), ns, P.ct.nvc, e.tl_mem,
                              e.tl_bytes, &K.pc32, st, reorder ? lab.data() : nullptr, P.agg_target, &h_seg_agg,
-                             &h_agg_ptr));
+                             &h_agg_rows));
   ClusterPlan cluster;
-  if (P.precond != kPrecTwoLevel || K.pc32.agg_contig)
+  if (P.precond != kPrecTwoLevel || h_agg_rows.size() == 2 * (size_t)h_seg_agg[ns])
     LAPY_TRY(cluster_plan(n, P.nnz, indptr, indices, e.k32, ns, P.ct.h_seg_row.data(),
-                          P.precond == kPrecTwoLevel ? h_seg_agg.data() : nullptr, h_agg_ptr.data(), p, e.sell_mem,
+                          P.precond == kPrecTwoLevel ? h_seg_agg.data() : nullptr, h_agg_rows.data(), p, e.sell_mem,
                           e.sell_bytes, &cluster, st));
   if (cluster.ok) {
     K.cluster = &cluster;

@@ -1053,7 +1053,7 @@ static int make_streams(ClusterPlan* plan) {
 
 // ---- planning ----------------------------------------------------------------------
 int cluster_plan(int64_t n, int64_t nnz, const int32_t* indptr, const int32_t* indices, const float* k32, int nseg,
-                 const int32_t* seg_row, const int32_t* seg_agg, const int32_t* agg_ptr, int p, void* mem,
+                 const int32_t* seg_row, const int32_t* seg_agg, const int32_t* agg_rows, int p, void* mem,
                  size_t bytes, ClusterPlan* out, cudaStream_t stream) {
   out->ok = false;
   const bool tl = seg_agg != nullptr;
@@ -1067,8 +1067,11 @@ int cluster_plan(int64_t n, int64_t nnz, const int32_t* indptr, const int32_t* i
     if (seg_row[s + 1] - seg_row[s] > 16 * kClMaxRows) return LAPY_OK;
     const bool has = tl && seg_agg[s + 1] > seg_agg[s];
     const int g0 = has ? seg_agg[s] : 0, g1 = has ? seg_agg[s + 1] : 1;
+    int32_t next = seg_row[s];  // the units of a segment cover its rows
     for (int g = g0; g < g1; ++g) {
-      const int32_t r0 = has ? agg_ptr[g] : seg_row[s], r1 = has ? agg_ptr[g + 1] : seg_row[s + 1];
+      const int32_t r0 = has ? agg_rows[2 * g] : seg_row[s], r1 = has ? agg_rows[2 * g + 1] : seg_row[s + 1];
+      if (r0 != next || r1 < r0) return LAPY_OK;
+      next = r1;
       if (has) agg_unit[2 * g] = (int32_t)unit_row.size();
       for (int32_t r = r0; r < r1; r += 32) {
         unit_row.push_back(r);
@@ -1076,6 +1079,7 @@ int cluster_plan(int64_t n, int64_t nnz, const int32_t* indptr, const int32_t* i
       }
       if (has) agg_unit[2 * g + 1] = (int32_t)unit_row.size();
     }
+    if (next != seg_row[s + 1]) return LAPY_OK;
   }
   const int nunit = (int)unit_row.size();
   seg_unit[nseg] = nunit;

@@ -59,12 +59,13 @@ struct ClusterPlan {
 };
 
 // Plan the clusters for p columns and build the packed FP32 matrix into
-// `mem`.  seg_agg / agg_ptr (host; null: Jacobi): aggregates per segment and
-// their row ranges, covering every row of a segment that has any.
-// out->ok = false (and nothing else) when a segment does not fit on chip, the
-// copy does not fit into `bytes`, or a column lies outside its segment.
+// `mem`.  seg_agg / agg_rows (host; null: Jacobi): aggregates per segment, and
+// the first row and the end of each.
+// out->ok = false (and nothing else) when a segment does not fit on chip, its
+// aggregates do not cover its rows one after the other, the copy does not fit
+// into `bytes`, or a column lies outside its segment.
 int cluster_plan(int64_t n, int64_t nnz, const int32_t* indptr, const int32_t* indices, const float* k32, int nseg,
-                 const int32_t* seg_row, const int32_t* seg_agg, const int32_t* agg_ptr, int p, void* mem,
+                 const int32_t* seg_row, const int32_t* seg_agg, const int32_t* agg_rows, int p, void* mem,
                  size_t bytes, ClusterPlan* out, cudaStream_t stream);
 
 struct ClusterSolve {
