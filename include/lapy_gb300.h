@@ -266,7 +266,9 @@ int lapy_csr_dirichlet_mask(int64_t n, const int32_t* indptr, const int32_t* ind
  * row-major n x ncol.  mixed != 0: FP32 Jacobi-PCG inside FP64 iterative
  * refinement (each round to inner_rtol); mixed == 0: FP64 Jacobi-PCG.
  * Stops when ||B - K X|| <= rtol ||B|| per (segment, column).
- * status_out / relres_out: host arrays nseg*ncol (row s*ncol + c). */
+ * status_out / relres_out: host arrays nseg*ncol (row s*ncol + c).  NaN or Inf
+ * in a column of B: LAPY_ERR_NAN and relres NaN for its mesh, the others as
+ * without it. */
 size_t lapy_pcg_solve_workspace_bytes(int64_t n, int64_t nnz, int nseg, const int32_t* seg_row,
                                       int ncol, int mixed);
 int lapy_pcg_solve(int64_t n, const int32_t* indptr, const int32_t* indices,

@@ -405,8 +405,24 @@ __global__ void __launch_bounds__(32 * kClMaxWarps, 1) ir_cluster_kernel(const C
     hb = reduce64(acc);
   }
 
-  int fst = LAPY_OK;  // column `lane` (boss warp)
-  bool masked = !(hb > 0.0);
+  // columns that are done, zeroed in R: solved, failed, or never begun (a zero
+  // right-hand side is solved by zero; NaN or Inf in it is an error, and its
+  // solution is left zero)
+  auto clear = [&](int mk) {
+#pragma unroll
+    for (int i = 0; i < UPW; ++i)
+#pragma unroll
+      for (int q = 0; q < NP; ++q)
+        if ((mk >> q) & 1) R[i][q] = 0.f;
+  };
+  int fst = isfinite(hb) ? LAPY_OK : LAPY_ERR_NAN;  // column `lane` (boss warp)
+  bool masked = !(hb > 0.0) || !isfinite(hb);
+  if (boss) {
+    const unsigned mk = __ballot_sync(0xffffffffu, lane >= NP || masked);
+    if (lane == 0) s_mask = (int)mk;
+  }
+  __syncthreads();
+  clear(s_mask);
   double round_rtol = a.inner_rtol;
   int iters = 0, rounds = 0;
   for (int round = 0; round < a.max_rounds; ++round) {
@@ -782,21 +798,16 @@ __global__ void __launch_bounds__(32 * kClMaxWarps, 1) ir_cluster_kernel(const C
       }
     }
     __syncthreads();
-    const int mk = s_mask;
     round_rtol = s_rtol;
     if (s_rdone) break;
-#pragma unroll
-    for (int i = 0; i < UPW; ++i)
-#pragma unroll
-      for (int q = 0; q < NP; ++q)
-        if ((mk >> q) & 1) R[i][q] = 0.f;
+    clear(s_mask);
   }
   if (rank == 0 && boss) {
     if (lane < NP) {
       const int64_t o = (int64_t)c.seg * a.p + c.col0 + lane;
       if (fst == LAPY_OK && hb > 0.0 && !(hr <= a.rtol * a.rtol * hb)) fst = LAPY_ERR_NOCONV;
       a.state[o] = fst;
-      a.relres2[o] = hb > 0.0 ? hr / hb : 0.0;
+      a.relres2[o] = !isfinite(hb) ? nan("") : hb > 0.0 ? hr / hb : 0.0;
     }
     if (lane == 0) {
       atomicMax(a.ctl + 0, (unsigned long long)iters);

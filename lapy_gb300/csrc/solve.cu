@@ -166,6 +166,7 @@ int ir_solve(const SysMatrix& K, const ChunkTable& ct, int p, const double* B, d
 
   std::vector<double> hb(nsp), hr(nsp);
   std::vector<int32_t> hst(nsp), hmask(nsp, 0), final_st(nsp, LAPY_OK);
+  auto relres2 = [&](int i) { return !std::isfinite(hb[i]) ? NAN : hb[i] > 0 ? hr[i] / hb[i] : 0.0; };
   LAPY_TRY(seg_col_norm2(B, p, ct, bn2, stream));
   LAPY_CUDA_TRY(cudaMemcpyAsync(hb.data(), bn2, sizeof(double) * nsp, cudaMemcpyDeviceToHost, stream));
   IrStats local;
@@ -186,7 +187,7 @@ int ir_solve(const SysMatrix& K, const ChunkTable& ct, int p, const double* B, d
     for (int i = 0; i < nsp; ++i) {
       if (hst[i] < 0) final_st[i] = hst[i];
       else if (hb[i] > 0 && !(hr[i] <= rtol * rtol * hb[i] * 1.0000001)) final_st[i] = LAPY_ERR_NOCONV;
-      if (relres2_host) relres2_host[i] = hb[i] > 0 ? hr[i] / hb[i] : 0.0;
+      if (relres2_host) relres2_host[i] = relres2(i);
     }
   } else if (K.reliable && K.pc32.kind == kPrecJacobi) {
     // one launch: FP32 iterations, FP64 solution and residual updates
@@ -204,20 +205,27 @@ int ir_solve(const SysMatrix& K, const ChunkTable& ct, int p, const double* B, d
     for (int i = 0; i < nsp; ++i) {
       if (hst[i] < 0) final_st[i] = hst[i];
       else if (hb[i] > 0 && !(hr[i] <= rtol * rtol * hb[i] * 1.0000001)) final_st[i] = LAPY_ERR_NOCONV;
-      if (relres2_host) relres2_host[i] = hb[i] > 0 ? hr[i] / hb[i] : 0.0;
+      if (relres2_host) relres2_host[i] = relres2(i);
     }
   } else {
     LAPY_CUDA_TRY(cudaMemsetAsync(X, 0, sizeof(double) * n * p, stream));
     LAPY_CUDA_TRY(cudaMemcpyAsync(R64, B, sizeof(double) * n * p, cudaMemcpyDeviceToDevice, stream));
     LAPY_CUDA_TRY(cudaStreamSynchronize(stream));
     bool done = false;
-    for (int i = 0; i < nsp; ++i) hmask[i] = !(hb[i] > 0);
+    // zero right-hand sides are solved by zero; NaN or Inf in one is an error,
+    // and its solution is left zero
+    bool bad = false;
+    for (int i = 0; i < nsp; ++i) {
+      hmask[i] = !(hb[i] > 0) || !std::isfinite(hb[i]);
+      if (!std::isfinite(hb[i])) final_st[i] = LAPY_ERR_NAN;
+      bad |= final_st[i] != LAPY_OK;
+    }
     // per-round FP32 target: at least inner_rtol, but only the reduction still
     // missing (with a factor 4 margin) once the residual is close to rtol
     double round_rtol = inner_rtol;
     for (int round = 0; round < max_rounds && !done; ++round) {
       LAPY_TRY(cast_f64_f32(n * p, R64, R32, stream));
-      if (round > 0) {
+      if (round > 0 || bad) {
         LAPY_CUDA_TRY(cudaMemcpyAsync(mask, hmask.data(), sizeof(int32_t) * nsp, cudaMemcpyHostToDevice, stream));
         mask_cols_kernel<<<ct.nchunk, 256, 0, stream>>>(R32, p, ct.chunk_row, ct.chunk_seg, mask);
         LAPY_TRY(lapy_check_launch("mask_cols_kernel"));
@@ -253,7 +261,7 @@ int ir_solve(const SysMatrix& K, const ChunkTable& ct, int p, const double* B, d
     }
     for (int i = 0; i < nsp; ++i) {
       if (final_st[i] == LAPY_OK && hb[i] > 0 && !(hr[i] <= rtol * rtol * hb[i])) final_st[i] = LAPY_ERR_NOCONV;
-      if (relres2_host) relres2_host[i] = hb[i] > 0 ? hr[i] / hb[i] : 0.0;
+      if (relres2_host) relres2_host[i] = relres2(i);
     }
   }
   int worst = LAPY_OK;
