@@ -1414,8 +1414,9 @@ static int eigs_run(const EigPlan& P, const EigPtrs& e, const int32_t* indptr, c
       for (int s = 0; s < ns; ++s) nact += hact[s] != 0;
       const double check_cost = kCheckSecPerDim * (double)(m + p) * (1.0 + (double)nact / kCheckMeshes);
       const double it = (double)step_pcg_iters;
-      const double step_cost = def.taken ? kChipStepSec + it * (kChipIterSec + kChipIterSecPerRow * (double)n)
-                                         : kGridStepSec + it * (kGridIterSec + kGridIterSecPerRow * (double)n);
+      // (by what solves: the profile's timers keep the solve from being deferred)
+      const double step_cost = cluster.ok ? kChipStepSec + it * (kChipIterSec + kChipIterSecPerRow * (double)n)
+                                          : kGridStepSec + it * (kGridIterSec + kGridIterSecPerRow * (double)n);
       const int balanced = (int)std::lround(std::sqrt(2.0 * check_cost / step_cost));
       const int steps = (int)std::lround((double)missing / std::max(1, nact) / (kPairsPerVector * p));
       int stride = std::max({1, steps, balanced});
