@@ -20,6 +20,7 @@
 #include "pcg.cuh"
 #include "blas.cuh"
 #include "scan.cuh"
+#include "slice_starts.h"
 
 namespace lapy {
 
@@ -1779,18 +1780,18 @@ int build_sell(int64_t n, const int32_t* indptr, const int32_t* indices, const V
   if (bytes < sell_bytes_bound(0, ct, sizeof(V))) return LAPY_OK;
   char* w = (char*)(((uintptr_t)mem + 255) & ~uintptr_t(255));
   char* end = (char*)mem + bytes;
-  int32_t* counts = (int32_t*)w; w += a256(4 * (size_t)(ct.nunit + 1));
-  int32_t* scratch = (int32_t*)w; w += a256(4 * (size_t)scan_scratch_elems(ct.nunit + 1));
   int32_t* slice_ptr = (int32_t*)w; w += a256(4 * (size_t)(ct.nunit + 1));
   const unsigned blocks = lapy_ceil_div((int64_t)ct.nunit * 32, 256);
-  sell_width_kernel<<<blocks, 256, 0, stream>>>(ct.nunit, ct.unit_row, indptr, counts);
+  sell_width_kernel<<<blocks, 256, 0, stream>>>(ct.nunit, ct.unit_row, indptr, slice_ptr);
   LAPY_TRY(lapy_check_launch("sell_width_kernel"));
-  LAPY_TRY(exclusive_scan_i32(counts, slice_ptr, ct.nunit, scratch, stream));
-  int32_t total = 0;
-  LAPY_CUDA_TRY(cudaMemcpyAsync(&total, slice_ptr + ct.nunit, sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
+  std::vector<int32_t> size((size_t)ct.nunit), starts;
+  LAPY_CUDA_TRY(cudaMemcpyAsync(size.data(), slice_ptr, 4 * (size_t)ct.nunit, cudaMemcpyDeviceToHost, stream));
   LAPY_CUDA_TRY(cudaStreamSynchronize(stream));
+  const int64_t total = slice_starts(size.data(), ct.nunit, &starts);
+  if (total < 0) return LAPY_OK;
   const size_t need = a256(4 * (size_t)total) + a256(sizeof(V) * (size_t)total);
-  if ((size_t)(end - w) < need || total < 0) return LAPY_OK;  // too much padding: the CSR path is used
+  if ((size_t)(end - w) < need) return LAPY_OK;  // too much padding: the CSR path is used
+  LAPY_CUDA_TRY(cudaMemcpyAsync(slice_ptr, starts.data(), 4 * starts.size(), cudaMemcpyHostToDevice, stream));
   int32_t* col = (int32_t*)w; w += a256(4 * (size_t)total);
   V* val = (V*)w;
   sell_fill_kernel<V><<<blocks, 256, 0, stream>>>(ct.nunit, ct.unit_row, indptr, indices, vals, slice_ptr, col, val);

@@ -38,6 +38,7 @@
 #include "fork_join.h"
 #include "pcg_cluster.cuh"
 #include "scan.cuh"
+#include "slice_starts.h"
 
 namespace lapy {
 
@@ -1209,7 +1210,7 @@ int cluster_plan(int64_t n, int64_t nnz, const int32_t* indptr, const int32_t* i
   auto* d_rank = (int32_t*)take(4 * (size_t)words);
   auto* d_scr = (int32_t*)take(4 * (size_t)scan_scratch_elems(nunit + 1));
   auto* d_cnt = (int32_t*)take(4 * (size_t)(nunit + 1));
-  // read back together: slices, push lists, halo sizes, flag
+  // read back together: slice sizes (summed there), push lists, halo sizes, flag
   auto* d_ptr = (int32_t*)take(4 * (size_t)(nunit + 1));
   auto* d_pp = (int32_t*)take(4 * (size_t)(nunit + 1));
   auto* d_halo = (int32_t*)take(4 * (size_t)nsplit);
@@ -1229,9 +1230,8 @@ int cluster_plan(int64_t n, int64_t nnz, const int32_t* indptr, const int32_t* i
   LAPY_TRY(put(d_aun, agg_unit.data(), 8 * (size_t)nagg));
   LAPY_CUDA_TRY(cudaMemsetAsync(d_bad, 0, 4, stream));
   const unsigned blocks = lapy_ceil_div((int64_t)nunit * 32, 256);
-  cl_width_kernel<<<blocks, 256, 0, stream>>>(nunit, d_row, d_uct, d_cu0, indptr, indices, d_cnt, d_slot);
+  cl_width_kernel<<<blocks, 256, 0, stream>>>(nunit, d_row, d_uct, d_cu0, indptr, indices, d_ptr, d_slot);
   LAPY_TRY(lapy_check_launch("cl_width_kernel"));
-  LAPY_TRY(exclusive_scan_i32(d_cnt, d_ptr, nunit, d_scr, stream));
   LAPY_CUDA_TRY(cudaMemsetAsync(d_cnt, 0, 4 * (size_t)(nunit + 1), stream));
   cl_halo_kernel<<<nsplit, 256, 0, stream>>>(d_spl, indptr, indices, d_slot, d_cu0, d_bits, d_rank, d_halo, d_cnt,
                                              d_bad);
@@ -1240,17 +1240,19 @@ int cluster_plan(int64_t n, int64_t nnz, const int32_t* indptr, const int32_t* i
   std::vector<char> hback(back);
   LAPY_CUDA_TRY(cudaMemcpyAsync(hback.data(), d_ptr, back, cudaMemcpyDeviceToHost, stream));
   LAPY_CUDA_TRY(cudaStreamSynchronize(stream));
-  const int32_t* slice = (const int32_t*)hback.data();
+  std::vector<int32_t> slice;
+  const int64_t total = slice_starts((const int32_t*)hback.data(), nunit, &slice);
   const int32_t* pptr = (const int32_t*)(hback.data() + ((char*)d_pp - (char*)d_ptr));
   const int32_t* halo = (const int32_t*)(hback.data() + ((char*)d_halo - (char*)d_ptr));
   if (*(const int*)(hback.data() + ((char*)d_bad - (char*)d_ptr))) return LAPY_OK;
-  const int64_t total = slice[nunit], npush = pptr[nunit];
-  if (total < 0 || npush < 0) return LAPY_OK;
+  const int64_t npush = pptr[nunit];  // (no more than the matrix has entries)
+  if (total < 0) return LAPY_OK;
   auto* d_push = (uint32_t*)take(4 * (size_t)npush);
   auto* d_code = (uint16_t*)take(2 * (size_t)total);
   auto* d_val = (float*)take(4 * (size_t)total);
   auto* d_diag = (float*)take(128 * (size_t)nunit);
   if (w > end) return LAPY_OK;
+  LAPY_TRY(put(d_ptr, slice.data(), 4 * slice.size()));
 
   // launches: clusters of one size together, the larger meshes first
   std::vector<int32_t> items(nseg);
