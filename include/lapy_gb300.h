@@ -354,6 +354,10 @@ int lapy_ic0_pcg_solve(int64_t n, const int32_t* indptr, const int32_t* indices,
  * evals: device nseg*k (ascending per segment); evecs: device row-major n x k,
  * M-orthonormal per segment.  status_out / nbasis_out: host nseg.
  * tol: Ritz residual tolerance; inner_rtol: inner-solve residual target.
+ * status_out[s]: LAPY_OK; LAPY_ERR_NOCONV after max_vectors; LAPY_ERR_BREAKDOWN
+ * when the blocks that fit into a mesh's rows do not reach tol (a mesh of a few
+ * blocks' rows, no multiple of the block: add uncoupled rows of far eigenvalues
+ * up to one).
  * precond: preconditioner of the inner PCG, LAPY_PRECOND_JACOBI or
  * LAPY_PRECOND_TWO_LEVEL (Jacobi plus a per-mesh aggregation coarse space
  * with a dense coarse inverse; the reference factorises instead, splu). */

@@ -541,8 +541,11 @@ __global__ void reorth_mask_kernel(int nseg, int p, const double* __restrict__ n
 // Cholesky of the p x p Gram matrix of every segment: G = R' R (R upper), one
 // warp per segment, lane i holding column i of R (p <= 16): a pivot's square
 // root and reciprocal are the chain, one of each per column (one thread did a
-// division per entry: 25 us at p = 8).  Inactive segments get R = I.
-// fail[s] = 1 when G is not numerically SPD.
+// division per entry: 25 us at p = 8).  Inactive segments get R = I.  A column
+// that depends on those before it to rounding is dropped: its row of R is zero,
+// and so are its columns of Q and of the projected matrix from there on (the
+// basis keeps the directions that are there, its Ritz values those of the rest).
+// fail[s] = 1 when no column is left: the basis holds an invariant space.
 __global__ void chol_small_kernel(int nseg, int p, const double* __restrict__ G, double* __restrict__ R,
                                   const int32_t* __restrict__ active, int32_t* __restrict__ fail) {
   const int s = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
@@ -560,14 +563,15 @@ __global__ void chol_small_kernel(int nseg, int p, const double* __restrict__ G,
   double col[16];  // rows j of column i, what is left of (G + G') / 2, then R
 #pragma unroll
   for (int j = 0; j < 16; ++j) col[j] = j < p ? 0.5 * (g[j * p + i] + g[i * p + j]) : 0.0;
-  int bad = 0;
+  int left = 0;
 #pragma unroll
   for (int j = 0; j < 16; ++j) {
     if (j < p) {
-      double d = __shfl_sync(0xffffffffu, col[j], j);
-      if (!(d > 1e-28 * gmax) || !isfinite(d)) { bad = 1; d = fmax(gmax, 1e-300) * 1e-28; }
-      const double rjj = sqrt(d), inv = 1.0 / rjj;
-      col[j] = i == j ? rjj : i > j ? col[j] * inv : 0.0;
+      const double d = __shfl_sync(0xffffffffu, col[j], j);
+      const bool keep = d > 1e-28 * gmax && isfinite(d);
+      const double rjj = keep ? sqrt(d) : 0.0, inv = keep ? 1.0 / rjj : 0.0;
+      left += keep;
+      col[j] = i == j ? rjj : i > j && keep ? col[j] * inv : 0.0;
 #pragma unroll
       for (int k = j + 1; k < 16; ++k)
         if (k < p) col[k] -= __shfl_sync(0xffffffffu, col[j], k) * col[j];
@@ -578,12 +582,13 @@ __global__ void chol_small_kernel(int nseg, int p, const double* __restrict__ G,
     for (int j = 0; j < 16; ++j)
       if (j < p) r[j * p + i] = col[j];
   }
-  if (lane == 0) fail[s] = bad;
+  if (lane == 0) fail[s] = left == 0;
 }
 
 // W(row, :) = W(row, :) * R_s^-1  (R upper triangular, p x p): R and the
 // reciprocals of its diagonal staged in shared memory once per chunk, so a
 // row costs p(p+1)/2 FMAs and no division (FP64 division is slow here).
+// Columns whose diagonal entry is zero become zero.
 template <int PT>
 __global__ void trsm_right_kernel(double* __restrict__ W, const double* __restrict__ R,
                                   const int32_t* __restrict__ chunk_row, const int32_t* __restrict__ chunk_seg) {
@@ -593,7 +598,10 @@ __global__ void trsm_right_kernel(double* __restrict__ W, const double* __restri
   const int s = chunk_seg[c];
   const double* r = R + (int64_t)s * PT * PT;
   for (int e = threadIdx.x; e < PT * PT; e += blockDim.x) sr[e] = r[e];
-  if (threadIdx.x < PT) sinv[threadIdx.x] = 1.0 / r[threadIdx.x * PT + threadIdx.x];
+  if (threadIdx.x < PT) {
+    const double d = r[threadIdx.x * PT + threadIdx.x];
+    sinv[threadIdx.x] = d == 0.0 ? 0.0 : 1.0 / d;
+  }
   __syncthreads();
   const int64_t r0 = chunk_row[c], r1 = chunk_row[c + 1];
   for (int64_t row = r0 + threadIdx.x; row < r1; row += blockDim.x) {
@@ -673,23 +681,23 @@ __global__ void copy_T_kernel(const double* __restrict__ T, double* __restrict__
   }
 }
 
-// Residual estimates of the k wanted Ritz pairs; freeze converged segments.
+// Residual estimates of the k wanted Ritz pairs; freeze converged segments, and
+// those whose rows the next block would not fit into: what it held beyond them
+// would be rounding noise, which Cholesky does not always flag.  nconv: pairs
+// that meet the tolerance, or -1 in a segment frozen without meeting it.
 __global__ void conv_check_kernel(int nseg, int p, int m, int lda, int keff, int k, double tol,
-                                  const double* __restrict__ theta, const double* __restrict__ S,
-                                  const double* __restrict__ Bm, const int32_t* __restrict__ fail,
+                                  const int32_t* __restrict__ seg_row, const double* __restrict__ theta,
+                                  const double* __restrict__ S, const double* __restrict__ Bm,
                                   int32_t* __restrict__ nconv, int32_t* __restrict__ active,
                                   double* __restrict__ Sfinal, double* __restrict__ theta_final,
                                   double* __restrict__ resid_out) {
   __shared__ double sh[32];
-  __shared__ int s_ok;
+  __shared__ int s_stop;
   const int s = blockIdx.x;
   if (!active[s]) return;
   const double* th = theta + (int64_t)s * keff;
   const double* Ss = S + (int64_t)s * lda * keff;
   const double* B = Bm + (int64_t)s * p * p;
-  // a rank-deficient new block means the Krylov space became invariant: the
-  // Ritz pairs are then exact and are accepted
-  const double tol_s = fail[s] ? 1e300 : tol;
   double worst = 0.0;
   int cnt = 0;
   for (int i = threadIdx.x; i < k; i += blockDim.x) {
@@ -700,8 +708,9 @@ __global__ void conv_check_kernel(int nseg, int p, int m, int lda, int keff, int
       r2 += v * v;
     }
     const double res = sqrt(r2) / fmax(fabs(th[i]), 1e-300);
-    worst = fmax(worst, isfinite(res) ? res : 1e300);
-    cnt += (res <= tol_s) ? 1 : 0;
+    const bool finite = isfinite(res) && isfinite(th[i]);
+    worst = fmax(worst, finite ? res : 1e300);
+    cnt += (finite && res <= tol) ? 1 : 0;
   }
   cnt = block_sum(cnt, (int*)sh);
   // block max
@@ -711,12 +720,13 @@ __global__ void conv_check_kernel(int nseg, int p, int m, int lda, int keff, int
   if (threadIdx.x == 0) {
     double w = 0.0;
     for (int i = 0; i < (int)(blockDim.x >> 5); ++i) w = fmax(w, sh[i]);
+    const bool ok = w <= tol, full = m + p > seg_row[s + 1] - seg_row[s];
     resid_out[s] = w;
-    nconv[s] = cnt;
-    s_ok = (w <= tol_s);
+    nconv[s] = ok || !full ? cnt : -1;
+    s_stop = ok || full;
   }
   __syncthreads();
-  if (!s_ok) return;
+  if (!s_stop) return;
   for (int64_t e = threadIdx.x; e < (int64_t)lda * keff; e += blockDim.x)
     Sfinal[(int64_t)s * lda * keff + e] = Ss[e];
   for (int i = threadIdx.x; i < keff; i += blockDim.x) theta_final[(int64_t)s * keff + i] = th[i];
@@ -1302,9 +1312,9 @@ static int eigs_run(const EigPlan& P, const EigPtrs& e, const int32_t* indptr, c
   res->status.assign(ns, LAPY_ERR_NOCONV);
   res->nbasis.assign(ns, 0);
   // First check once the basis holds ~2.5 k vectors (shift-invert Lanczos
-  // needs 3-5 k); afterwards the stride is the larger of (a) the block steps
-  // that the missing pairs take, on the mean over the unconverged meshes, and
-  // (b) the stride that balances the cost of a check c against that of a block
+  // needs 3-5 k), or the next block does not fit into the rows of the smallest
+  // mesh; afterwards the stride is the larger of (a) the block steps that the
+  // missing pairs take, on the mean over the unconverged meshes, and (b) the stride that balances the cost of a check c against that of a block
   // step s: checking every m steps costs c/m per step and overshoots
   // convergence by (m-1)/2 steps on average, least at m = sqrt(2 c / s).  c and
   // s come from a cost model of this GPU, not from timers, so the stopping
@@ -1313,6 +1323,8 @@ static int eigs_run(const EigPlan& P, const EigPtrs& e, const int32_t* indptr, c
   // and 11 instead of 6 for 128 meshes.)
   const int first_check = std::max((keff + p + p - 1) / p, (int)std::ceil(2.5 * k / p));
   int next_check = first_check;
+  int64_t rows_min = INT64_MAX;  // of the meshes that have not stopped
+  for (int s = 0; s < ns; ++s) rows_min = std::min<int64_t>(rows_min, P.ct.h_seg_row[s + 1] - P.ct.h_seg_row[s]);
   int64_t step_pcg_iters = 0;
   std::vector<int32_t> hnconv(ns);
   auto inner_done = [&](int status, int64_t iters) -> int {
@@ -1368,7 +1380,7 @@ static int eigs_run(const EigPlan& P, const EigPtrs& e, const int32_t* indptr, c
     LAPY_TRY(ops.chol_qr2(Qn));
     LAPY_TRY(ops.basis_to_df(j + 1));
     const int m = (j + 1) * p;
-    const bool check = (j + 1 >= next_check) || j + 1 == P.mb;
+    const bool check = (j + 1 >= next_check) || j + 1 == P.mb || rows_min < (int64_t)(j + 2) * p;
     bool any_fail = false;
     if (def.taken) {
       StepStatus hs;
@@ -1389,7 +1401,7 @@ static int eigs_run(const EigPlan& P, const EigPtrs& e, const int32_t* indptr, c
       copy_T_kernel<<<ns, 256, 0, st>>>(e.T, e.Tc, lda, m, e.active);
       LAPY_TRY(lapy_check_launch("copy_T_kernel"));
       LAPY_TRY(sym_eig_top(ns, e.Tc, lda, e.nsize, m, keff, e.theta, e.S, e.eigw, e.active, false, st));
-      conv_check_kernel<<<ns, 128, 0, st>>>(ns, p, m, lda, keff, k, tol, e.theta, e.S, e.Bm, e.fail, e.nconv,
+      conv_check_kernel<<<ns, 128, 0, st>>>(ns, p, m, lda, keff, k, tol, P.ct.seg_row, e.theta, e.S, e.Bm, e.nconv,
                                             e.active, e.Sfinal, e.theta_final, e.resid);
       LAPY_TRY(lapy_check_launch("conv_check_kernel"));
       std::vector<int32_t> hact2(ns);
@@ -1399,9 +1411,12 @@ static int eigs_run(const EigPlan& P, const EigPtrs& e, const int32_t* indptr, c
       all_done = true;
       int64_t missing = 0;
       int worst = 0;
-      int64_t rows_min = INT64_MAX;
+      rows_min = INT64_MAX;
       for (int s = 0; s < ns; ++s) {
-        if (hact[s] && !hact2[s]) { res->status[s] = LAPY_OK; res->nbasis[s] = m; }
+        if (hact[s] && !hact2[s]) {
+          res->status[s] = hnconv[s] < 0 ? LAPY_ERR_BREAKDOWN : LAPY_OK;
+          res->nbasis[s] = m;
+        }
         if (hact2[s]) {
           missing += k - hnconv[s];
           worst = std::max(worst, k - hnconv[s]);
@@ -1420,14 +1435,8 @@ static int eigs_run(const EigPlan& P, const EigPtrs& e, const int32_t* indptr, c
       const int balanced = (int)std::lround(std::sqrt(2.0 * check_cost / step_cost));
       const int steps = (int)std::lround((double)missing / std::max(1, nact) / (kPairsPerVector * p));
       int stride = std::max({1, steps, balanced});
-      // a basis that nears the rows of a mesh: short strides, and a check no
-      // later than the last block that fits (what a block adds beyond that is
-      // rounding noise, which Cholesky does not always flag)
-      if (rows_min < 2 * (int64_t)(j + 1 + stride) * p) {
-        stride = std::max(1, (worst + 2 * p - 1) / (2 * p));
-        const int64_t fits = rows_min / p;
-        if (fits > j + 1) stride = (int)std::min<int64_t>(stride, fits - (j + 1));
-      }
+      // a basis that nears the rows of a mesh: short strides
+      if (rows_min < 2 * (int64_t)(j + 1 + stride) * p) stride = std::max(1, (worst + 2 * p - 1) / (2 * p));
       next_check = j + 1 + stride;
     }
   }

@@ -11,7 +11,7 @@ import torch
 
 from . import _lib
 from ._device import DeviceCSR, MeshDevice, assemble, build_pattern, dptr, require_cuda, stream
-from .solver import DEFAULT_BLOCK, Solver, eigs_batched
+from .solver import DEFAULT_BLOCK, Solver, eigs_batched, eigs_filled
 
 
 def _ev_dict(geom, k, evals, evecs) -> dict:
@@ -195,7 +195,16 @@ def compute_shapedna_batch(meshes, k: int = 50, lump: bool = False, block: int =
         tuning = autotune.solver_tuning(choice)
     batch = BatchedFEM(meshes, lump=lump)
     evals, evecs, info = batch.eigs(k=k, block=block, tuning=tuning, **kw)
-    bad = [int(s) for s in info["status"] if s != 0]
+    status = np.array(info["status"])
+    for i in np.nonzero(status == _lib.ERR_BREAKDOWN)[0]:  # a mesh of a few blocks' rows, by itself
+        r0, r1 = batch.seg_row[i], batch.seg_row[i + 1]
+        one = BatchedFEM([meshes[i]], lump=lump)
+        evals[i:i + 1], evecs[r0:r1], alone = eigs_filled(one.indptr, one.indices, one.a_vals, one.m_vals,
+                                                          one.m_is_diag, one.n, k, kw.get("sigma", -0.01), block,
+                                                          tuning=tuning,
+                                                          **{key: val for key, val in kw.items() if key != "sigma"})
+        status[i] = alone["status"][0]
+    bad = [int(s) for s in status if s != 0]
     if bad:
         _lib.check(bad[0], "compute_shapedna_batch")
     ev = evals.cpu().numpy()

@@ -157,9 +157,12 @@ class Solver:
         block = block or DEFAULT_BLOCK
         while block > 1 and n < k + 2 * block + 1:
             block //= 2
-        evals, evecs, info = eigs_batched(A.indptr, A.indices, A.data.contiguous(), mvals, m_diag,
-                                          np.array([0, n], dtype=np.int32), k, sigma, block, tol, inner_rtol,
+        system = (A.indptr, A.indices, A.data.contiguous(), mvals, m_diag)
+        evals, evecs, info = eigs_batched(*system, np.array([0, n], dtype=np.int32), k, sigma, block, tol, inner_rtol,
                                           precond=precond)
+        if int(info["status"][0]) == _lib.ERR_BREAKDOWN:
+            evals, evecs, info = eigs_filled(*system, n, k, sigma, block, tol=tol, inner_rtol=inner_rtol,
+                                             precond=precond)
         st = int(info["status"][0])
         if st != 0:
             _lib.check(st, "Solver.eigs")
@@ -297,3 +300,26 @@ def eigs_batched(indptr, indices, a_vals, m_vals, m_is_diag: bool, seg_row, k: i
     info = {"status": status, "nbasis": nbasis, "inner_iters": int(iters.value), "block": block, "precond": precond,
             "workspace_bytes": int(ws_bytes), "tuning": dict(tuning or {})}
     return evals, evecs, info
+
+
+def eigs_filled(indptr, indices, a_vals, m_vals, m_is_diag: bool, n: int, k: int, sigma: float, block: int,
+                max_vectors: int | None = None, **kw):
+    """``eigs_batched`` of one mesh whose rows the blocks do not fill, where it
+    needs all of them: with uncoupled rows added up to a multiple of ``block``,
+    of eigenvalues far beyond the mesh's, so that the basis can hold the whole
+    space.  (Narrower blocks would fit too, but miss copies of eigenvalues that
+    have more of them than a block has columns.)"""
+    pad = -n % block
+    more = torch.arange(n, n + pad, dtype=indices.dtype, device=indices.device)
+    ip = torch.cat((indptr, indptr[-1] + 1 + torch.arange(pad, dtype=indptr.dtype, device=indptr.device)))
+    rows = torch.repeat_interleave(torch.arange(n, device=indices.device), indptr.diff().long())
+    on_diag = rows == indices
+    m_diag = m_vals[rows[on_diag]] if m_is_diag else m_vals[on_diag]
+    mass = m_diag.mean().expand(pad)
+    far = 100.0 * (a_vals[on_diag] / m_diag).max()
+    stiff = far * mass * (1.0 + torch.arange(pad, dtype=a_vals.dtype, device=a_vals.device))
+    evals, evecs, info = eigs_batched(ip, torch.cat((indices, more)), torch.cat((a_vals, stiff)),
+                                      torch.cat((m_vals, mass)), m_is_diag, np.array([0, n + pad], dtype=np.int32), k,
+                                      sigma, block, max_vectors=max(max_vectors or 6 * k + 8 * block, n + pad + block),
+                                      **kw)
+    return evals, evecs[:n].contiguous(), info
