@@ -1314,13 +1314,17 @@ static int eigs_run(const EigPlan& P, const EigPtrs& e, const int32_t* indptr, c
   // First check once the basis holds ~2.5 k vectors (shift-invert Lanczos
   // needs 3-5 k), or the next block does not fit into the rows of the smallest
   // mesh; afterwards the stride is the larger of (a) the block steps that the
-  // missing pairs take, on the mean over the unconverged meshes, and (b) the stride that balances the cost of a check c against that of a block
-  // step s: checking every m steps costs c/m per step and overshoots
-  // convergence by (m-1)/2 steps on average, least at m = sqrt(2 c / s).  c and
-  // s come from a cost model of this GPU, not from timers, so the stopping
-  // step - and with it every result - is the same on every run.  (With half of
-  // the missing pairs' blocks as (a), 10 checks instead of 5 for 642 vertices
-  // and 11 instead of 6 for 128 meshes.)
+  // missing pairs take, on the mean over the unconverged meshes, and (b) the
+  // stride that balances the cost of a check c against that of a block step s:
+  // checking every m steps costs c/m per step and overshoots convergence by
+  // (m-1)/2 steps on average, least at m = sqrt(2 c / s).  c and s come from a
+  // cost model of this GPU, not from timers, so the stopping step - and with it
+  // every result - is the same on every run.  (With half of the missing pairs'
+  // blocks as (a), 10 checks instead of 5 for 642 vertices and 11 instead of 6
+  // for 128 meshes.)  No more pairs than a block has columns are checked at
+  // every step: where an eigenvalue has more copies than that, rounding brings
+  // the others into the basis later, and the first ones look unconverged while
+  // they mix.
   const int first_check = std::max((keff + p + p - 1) / p, (int)std::ceil(2.5 * k / p));
   int next_check = first_check;
   int64_t rows_min = INT64_MAX;  // of the meshes that have not stopped
@@ -1434,7 +1438,7 @@ static int eigs_run(const EigPlan& P, const EigPtrs& e, const int32_t* indptr, c
                                           : kGridStepSec + it * (kGridIterSec + kGridIterSecPerRow * (double)n);
       const int balanced = (int)std::lround(std::sqrt(2.0 * check_cost / step_cost));
       const int steps = (int)std::lround((double)missing / std::max(1, nact) / (kPairsPerVector * p));
-      int stride = std::max({1, steps, balanced});
+      int stride = k <= p ? 1 : std::max({1, steps, balanced});
       // a basis that nears the rows of a mesh: short strides
       if (rows_min < 2 * (int64_t)(j + 1 + stride) * p) stride = std::max(1, (worst + 2 * p - 1) / (2 * p));
       next_check = j + 1 + stride;

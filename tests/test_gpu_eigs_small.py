@@ -83,3 +83,14 @@ def test_symmetric_mesh(cuda_ok, level, k):
     m = meshes.icosphere(level)
     got, _ = Solver(m).eigs(k=k)
     assert _close(got, _want(m, k))
+
+
+def test_pieces_that_all_have_a_constant(cuda_ok):
+    """Twelve disjoint patches: zero is there twelve times, a block finds as many as it has columns."""
+    from lapy_gb300 import shapedna
+    from test_gpu_coarse_edge import _pieces
+
+    for block in (1, 2, 4, 8):
+        evals, _, info = shapedna.BatchedFEM([_pieces()]).eigs(k=block, block=block)
+        assert int(info["status"][0]) == 0
+        assert np.all(np.abs(evals.cpu().numpy()) <= 1.01e-10)
