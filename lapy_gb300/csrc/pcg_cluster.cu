@@ -13,7 +13,7 @@
 // they are read (p = z + beta p; their owners store z), so that r'z is reduced
 // by the barrier that publishes z and q = K p, p'q are computed as plain CG
 // has them: three cluster barriers per iteration with the two-level
-// preconditioner, two with Jacobi.  (The Chronopoulos-Gear form, q by recurrence
+// preconditioner, two with Jacobi (one more where the copies are many).  (The Chronopoulos-Gear form, q by recurrence
 // and p'q = z'K z - beta r'z / alpha_old, needs no more barriers either, but the
 // difference cancels where K is close to singular in FP32: spheres of radius
 // 0.02 and 0.03 at sigma = -0.01 took up to 25 times the iterations or failed.)
@@ -48,6 +48,12 @@ constexpr int kClMaxWarps = 16;
 constexpr int kClMaxRows = 4096;  // rows per CTA a 12-bit code can name
 constexpr size_t kClSmemMax = 226 * 1024;  // dynamic; the rest of the 227 KB is static
 constexpr int32_t kClActive = INT32_MAX;
+// Most halo rows whose directions a CTA updates itself, from copies of z.  More
+// of them, or copies that do not fit, are sent as directions, after one more
+// barrier: 390 and 2,023 rows a CTA are 9 and 3 % slower that way (geodesics of
+// 40,962 vertices, eigs of 11,466), 15,348 rows 17 % faster (Poisson on 40,962
+// vertices in the order of refinement: 11.9 -> 9.9 ms).
+constexpr int kZHalo = 5000;
 
 struct ClArgs {
   int p;
@@ -77,7 +83,7 @@ struct ClArgs {
   int32_t* state;
   double* relres2;
   unsigned long long* ctl;
-  int mat_smem, coarse_smem;
+  int mat_smem, coarse_smem, z_halo;
   // shared memory layout (byte offsets, the same in every CTA of a launch) and
   // rows reserved for the halo's z and for p (own rows and halo)
   int o_z, o_p, o_rc, o_yc, o_up, o_wp, o_mail, o_tab, o_push, o_val, o_code, o_coarse;
@@ -246,6 +252,7 @@ __global__ void __launch_bounds__(32 * kClMaxWarps, 1) ir_cluster_kernel(const C
   extern __shared__ __align__(16) unsigned char sm[];
   __shared__ float s_vrc[NP];
   __shared__ double s_rtol;
+  __shared__ int s_own[16];  // rows of every CTA's own slots
   __shared__ int s_act, s_rdone, s_mask;
   const ClusterCta c = a.cta[cta_base + blockIdx.x];
   const unsigned rank = cl_rank(), cs = cl_size();
@@ -309,6 +316,10 @@ __global__ void __launch_bounds__(32 * kClMaxWarps, 1) ir_cluster_kernel(const C
       aunit[g] = (ua - c.unit0) | ((ub - ua) << 16);
     }
   for (int i = threadIdx.x; i < h1 - h0; i += blockDim.x) push[i] = a.push[h0 + i];
+  if (threadIdx.x < cs) {
+    const ClusterCta* o = a.cta + cta_base + blockIdx.x - rank + threadIdx.x;
+    s_own[threadIdx.x] = 32 * (o->unit1 - o->unit0);
+  }
   for (int i = threadIdx.x; i < 16 * 5 * NP; i += blockDim.x) wp[i] = 0.f;    // all three areas
   for (int i = threadIdx.x; i < 16 * 7 * NP; i += blockDim.x) mail[i] = 0.f;  // all four areas
   const float* val = a.val + e0;
@@ -351,6 +362,36 @@ __global__ void __launch_bounds__(32 * kClMaxWarps, 1) ir_cluster_kernel(const C
       const float s = sum16(part + v, nv);
       if (dst == (int)rank) area[rank * nv + v] = s;
       else cl_store(cl_map(smem_u32(area + rank * nv + v), dst), s);
+    }
+  };
+  // this warp's rows into the neighbours' copies of them: rows of `arr` there,
+  // behind its own slots (own = 1) or by themselves (0)
+  auto push_rows = [&](const float (&v)[UPW][NP], float* arr, int plane, int own) {
+#pragma unroll
+    for (int i = 0; i < UPW; ++i) {
+      if (i < nu) {
+        const int e1 = upush[u0 + i + 1];
+        for (int e0 = upush[u0 + i]; e0 < e1; e0 += 32) {
+          const unsigned w = push[min(e0 + lane, e1 - 1)];  // slot (12 bits), rank (4), halo row (16)
+          const unsigned rk = (w >> 12) & 15u, dst = (w >> 16) + (unsigned)(own * s_own[rk]);
+          float x[NP];
+#pragma unroll
+          for (int q = 0; q < NP; ++q) x[q] = __shfl_sync(0xffffffffu, v[i][q], (int)(w & 31u));
+          if (e0 + lane < e1) {
+            const unsigned ra = cl_map(smem_u32(arr), rk);
+            if constexpr (NP >= 4) {
+#pragma unroll
+              for (int h = 0; h < NP / 4; ++h)
+                cl_store4(ra + 4u * (unsigned)(h * plane) + 16u * dst, x[4 * h], x[4 * h + 1], x[4 * h + 2],
+                          x[4 * h + 3]);
+            } else if constexpr (NP == 2) {
+              cl_store2(ra + 8u * dst, x[0], x[1]);
+            } else {
+              cl_store(ra + 4u * dst, x[0]);
+            }
+          }
+        }
+      }
     }
   };
   auto total = [&](const float* part, const float* area, int nv) -> float {
@@ -565,34 +606,7 @@ __global__ void __launch_bounds__(32 * kClMaxWarps, 1) ir_cluster_kernel(const C
         const float t = lane_totals<NV>(red);
         if (lane % per == 0) wp2[warp * NV + lane / per] = t;
       }
-      if (cs > 1) {  // copies for the neighbours (this warp's rows)
-#pragma unroll
-        for (int i = 0; i < UPW; ++i) {
-          if (i < nu) {
-            const int e1 = upush[u0 + i + 1];
-            for (int e0 = upush[u0 + i]; e0 < e1; e0 += 32) {
-              const unsigned w = push[min(e0 + lane, e1 - 1)];  // slot (12 bits), rank (4), halo row (16)
-              const unsigned dst = w >> 16, rk = (w >> 12) & 15u;
-              float x[NP];
-#pragma unroll
-              for (int q = 0; q < NP; ++q) x[q] = __shfl_sync(0xffffffffu, z[i][q], (int)(w & 31u));
-              if (e0 + lane < e1) {
-                const unsigned ra = cl_map(smem_u32(Z), rk);
-                if constexpr (NP >= 4) {
-#pragma unroll
-                  for (int h = 0; h < NP / 4; ++h)
-                    cl_store4(ra + 4u * (unsigned)(h * zplane) + 16u * dst, x[4 * h], x[4 * h + 1], x[4 * h + 2],
-                              x[4 * h + 3]);
-                } else if constexpr (NP == 2) {
-                  cl_store2(ra + 8u * dst, x[0], x[1]);
-                } else {
-                  cl_store(ra + 4u * dst, x[0]);
-                }
-              }
-            }
-          }
-        }
-      }
+      if (a.z_halo) push_rows(z, Z, zplane, 0);
       exchange(wp2, mail2, NV);
       if (cs > 1) cl_sync(cs);
       // ---- beta, p = z + beta p in the CTA's rows and its copies (scalars of
@@ -623,20 +637,25 @@ __global__ void __launch_bounds__(32 * kClMaxWarps, 1) ir_cluster_kernel(const C
             float pv[NP];
             cl_load<NP>(P, pplane, slot0 + 32 * i, pv);
 #pragma unroll
-            for (int q = 0; q < NP; ++q) pv[q] = fmaf(be[q], pv[q], z[i][q]);
-            cl_save<NP>(P, pplane, slot0 + 32 * i, pv);
+            for (int q = 0; q < NP; ++q) z[i][q] = fmaf(be[q], pv[q], z[i][q]);
+            cl_save<NP>(P, pplane, slot0 + 32 * i, z[i]);
           }
         }
-        for (int h = threadIdx.x; h < c.nhalo; h += blockDim.x) {
-          float zv[NP], pv[NP];
-          cl_load<NP>(Z, zplane, h, zv);
-          cl_load<NP>(P, pplane, 32 * nunit + h, pv);
+        if (a.z_halo) {
+          for (int h = threadIdx.x; h < c.nhalo; h += blockDim.x) {
+            float zv[NP], pv[NP];
+            cl_load<NP>(Z, zplane, h, zv);
+            cl_load<NP>(P, pplane, 32 * nunit + h, pv);
 #pragma unroll
-          for (int q = 0; q < NP; ++q) pv[q] = fmaf(be[q], pv[q], zv[q]);
-          cl_save<NP>(P, pplane, 32 * nunit + h, pv);
+            for (int q = 0; q < NP; ++q) pv[q] = fmaf(be[q], pv[q], zv[q]);
+            cl_save<NP>(P, pplane, 32 * nunit + h, pv);
+          }
+          __syncthreads();
+        } else {
+          if (cs > 1) push_rows(z, P, pplane, 1);
+          cl_sync(cs);
         }
       }
-      __syncthreads();
       // ---- q = K p, p'q
       float Q[UPW][NP];
       {
@@ -997,7 +1016,7 @@ static int max_units(int np) {
 }
 
 // Shared memory of a class; the byte offsets when `a` is given.
-static size_t class_layout(const ClusterClass& k, int np, bool tl, bool mat, bool coarse, ClArgs* a) {
+static size_t class_layout(const ClusterClass& k, int np, bool tl, bool mat, bool coarse, bool z_halo, ClArgs* a) {
   size_t off = 0;
   auto take = [&](size_t bytes) {
     const size_t o = off;
@@ -1005,7 +1024,7 @@ static size_t class_layout(const ClusterClass& k, int np, bool tl, bool mat, boo
     return (int)o;
   };
   const size_t row = 4 * (size_t)np;
-  const int zrows = k.halo, prows = k.slots;
+  const int zrows = z_halo ? k.halo : 0, prows = k.slots;
   const int oz = take(row * zrows), op = take(row * prows);
   const int orc = take(tl ? row * k.ld : 0), oyc = take(tl ? row * std::max(k.aggs, 1) : 0);
   const int oup = take(tl ? row * k.units : 0);
@@ -1307,9 +1326,10 @@ int cluster_plan(int64_t n, int64_t nnz, const int32_t* indptr, const int32_t* i
     if (!var) return LAPY_OK;
     k.kernel = (const void*)(tl ? var->tl : var->jacobi);
     k.warps = std::max(1, std::min(kClMaxWarps, k.units));
-    k.mat_smem = class_layout(k, np, tl, true, false, nullptr) <= kClSmemMax;
-    k.coarse_smem = class_layout(k, np, tl, k.mat_smem, true, nullptr) <= kClSmemMax;
-    k.smem = class_layout(k, np, tl, k.mat_smem, k.coarse_smem, nullptr);
+    k.z_halo = k.halo <= kZHalo && class_layout(k, np, tl, false, false, true, nullptr) <= kClSmemMax;
+    k.mat_smem = class_layout(k, np, tl, true, false, k.z_halo, nullptr) <= kClSmemMax;
+    k.coarse_smem = class_layout(k, np, tl, k.mat_smem, true, k.z_halo, nullptr) <= kClSmemMax;
+    k.smem = class_layout(k, np, tl, k.mat_smem, k.coarse_smem, k.z_halo, nullptr);
     if (k.smem > kClSmemMax) return LAPY_OK;
     LAPY_CUDA_TRY(cudaFuncSetAttribute(k.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClSmemMax));
     LAPY_CUDA_TRY(cudaFuncSetAttribute(k.kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
@@ -1388,7 +1408,8 @@ int cluster_solve(const ClusterPlan& plan, const ClusterSolve& s, cudaStream_t s
     const ClusterClass& k = plan.cls[i];
     cudaStream_t on = fork ? plan.streams[i] : stream;
     if (fork) LAPY_CUDA_TRY(cudaStreamWaitEvent(on, plan.events.back(), 0));
-    class_layout(k, plan.np, tl, k.mat_smem, k.coarse_smem, &a);
+    class_layout(k, plan.np, tl, k.mat_smem, k.coarse_smem, k.z_halo, &a);
+    a.z_halo = k.z_halo ? 1 : 0;
     a.mat_smem = k.mat_smem ? 1 : 0;
     a.coarse_smem = k.coarse_smem ? 1 : 0;
     cudaLaunchConfig_t cfg{};

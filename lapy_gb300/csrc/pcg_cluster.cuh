@@ -27,6 +27,7 @@ struct ClusterClass {
   int cta0 = 0, ncta = 0;
   int slots = 0, halo = 0, units = 0, aggs = 0, ld = 0, push = 0;  // largest of the class
   int64_t elems = 0;
+  bool z_halo = true;    // owners store z into the halo (else p, after one more barrier)
   bool mat_smem = true;  // matrix in shared memory (else read through L2)
   bool coarse_smem = true;  // rows of the coarse inverse likewise
   size_t smem = 0;
