@@ -242,6 +242,11 @@ __device__ __forceinline__ void cl_coarse(const uint16_t* kseg, int nc, int nrow
   }
 }
 
+template <int N>
+struct Count {
+  static constexpr int value = N;
+};
+
 // One cluster solves one segment's columns [col0, col0 + NP).  UPW: most
 // 32-row units a warp holds.  A CTA keeps its rows in slots of 32 per unit
 // (lanes past a unit's last row hold zero residuals and matrix entries, so the
@@ -343,7 +348,7 @@ __global__ void __launch_bounds__(32 * kClMaxWarps, 1) ir_cluster_kernel(const C
   }
   __syncthreads();
 
-  float R[UPW][NP], X[UPW][NP], dv[UPW], dg[UPW];
+  float R[UPW][NP], X[UPW][NP], D[UPW][NP], dv[UPW], dg[UPW];  // residual, solution, direction
   // global row of unit i of this warp and lane, or -1 past the unit's last row
   auto row_of = [&](int i) -> int64_t {
     if (i >= nu) return -1;
@@ -394,8 +399,19 @@ __global__ void __launch_bounds__(32 * kClMaxWarps, 1) ir_cluster_kernel(const C
       }
     }
   };
-  auto total = [&](const float* part, const float* area, int nv) -> float {
-    return lane >= nv ? 0.f : sum16((cs == 1 ? part : area) + lane, nv);
+  // value lane mod nv of the totals; nv = 1, 2, 4, 8 or 16, in every warp: all
+  // lanes read (16 reads by nv lanes of each warp took 512 of an iteration's
+  // shared-memory wavefronts)
+  auto total = [&](const float* part, const float* area, auto nvc) -> float {
+    constexpr int nv = decltype(nvc)::value;
+    const float* src = (cs == 1 ? part : area) + lane;
+    float v = 0.f;
+#pragma unroll
+    for (int j = 0; j < 16 * nv; j += 32)
+      if (16 * nv >= 32 || lane < 16 * nv) v += src[j];
+#pragma unroll
+    for (int m = 16; m >= nv; m >>= 1) v += __shfl_xor_sync(0xffffffffu, v, m);
+    return v;
   };
   // column sums over the cluster in FP64, on lanes 0..NP-1 of the boss warp
   auto reduce64 = [&](double (&acc)[NP]) -> double {
@@ -472,12 +488,9 @@ __global__ void __launch_bounds__(32 * kClMaxWarps, 1) ir_cluster_kernel(const C
     const float rtol2 = (float)(round_rtol * round_rtol);
     // ---- FP32 PCG from zero on R
 #pragma unroll
-    for (int i = 0; i < UPW; ++i) {
-      float zero[NP];
+    for (int i = 0; i < UPW; ++i)
 #pragma unroll
-      for (int q = 0; q < NP; ++q) { X[i][q] = 0.f; zero[q] = 0.f; }
-      if (i < nu) cl_save<NP>(P, pplane, slot0 + 32 * i, zero);
-    }
+      for (int q = 0; q < NP; ++q) { X[i][q] = 0.f; D[i][q] = 0.f; }
     for (int h = threadIdx.x; h < c.nhalo; h += blockDim.x) {
       float zero[NP];
 #pragma unroll
@@ -564,7 +577,7 @@ __global__ void __launch_bounds__(32 * kClMaxWarps, 1) ir_cluster_kernel(const C
         }
         cl_sync(cs);
         if (boss) {
-          const float s = total(wp, mail, 2 * NP);
+          const float s = total(wp, mail, Count<2 * NP>());
           if (lane >= NP && lane < 2 * NP) s_vrc[lane - NP] = cscale * s;
           if (lane < NP) judge(s);
           const unsigned m = __ballot_sync(0xffffffffu, lane < NP && st == kClActive);
@@ -611,7 +624,7 @@ __global__ void __launch_bounds__(32 * kClMaxWarps, 1) ir_cluster_kernel(const C
       if (cs > 1) cl_sync(cs);
       // ---- beta, p = z + beta p in the CTA's rows and its copies (scalars of
       // column `lane` in every warp)
-      float gam = total(wp2, mail2, NV);
+      float gam = total(wp2, mail2, Count<NV>());
       bool act;
       if constexpr (TL) {
         act = (s_act >> lane) & 1;
@@ -634,11 +647,9 @@ __global__ void __launch_bounds__(32 * kClMaxWarps, 1) ir_cluster_kernel(const C
 #pragma unroll
         for (int i = 0; i < UPW; ++i) {
           if (i < nu) {
-            float pv[NP];
-            cl_load<NP>(P, pplane, slot0 + 32 * i, pv);
 #pragma unroll
-            for (int q = 0; q < NP; ++q) z[i][q] = fmaf(be[q], pv[q], z[i][q]);
-            cl_save<NP>(P, pplane, slot0 + 32 * i, z[i]);
+            for (int q = 0; q < NP; ++q) D[i][q] = fmaf(be[q], D[i][q], z[i][q]);
+            cl_save<NP>(P, pplane, slot0 + 32 * i, D[i]);
           }
         }
         if (a.z_halo) {
@@ -652,7 +663,7 @@ __global__ void __launch_bounds__(32 * kClMaxWarps, 1) ir_cluster_kernel(const C
           }
           __syncthreads();
         } else {
-          if (cs > 1) push_rows(z, P, pplane, 1);
+          if (cs > 1) push_rows(D, P, pplane, 1);
           cl_sync(cs);
         }
       }
@@ -701,12 +712,10 @@ __global__ void __launch_bounds__(32 * kClMaxWarps, 1) ir_cluster_kernel(const C
                 Q[i][q] = fmaf(va.y, x1[q], Q[i][q]);
               }
             }
-            float pv[NP];
-            cl_load<NP>(P, pplane, slot0 + 32 * i, pv);
 #pragma unroll
             for (int q = 0; q < NP; ++q) {
-              Q[i][q] = fmaf(dg[i], pv[q], Q[i][q]);
-              red[q] = fmaf(pv[q], Q[i][q], red[q]);
+              Q[i][q] = fmaf(dg[i], D[i][q], Q[i][q]);
+              red[q] = fmaf(D[i][q], Q[i][q], red[q]);
             }
           }
         }
@@ -718,7 +727,7 @@ __global__ void __launch_bounds__(32 * kClMaxWarps, 1) ir_cluster_kernel(const C
       if (cs > 1) cl_sync(cs);
       // ---- x += alpha p, r -= alpha q
       {
-        const float pq = total(wp3, mail3, NP);
+        const float pq = total(wp3, mail3, Count<NP>());
         float alpha = 0.f;
         if (act) {
           if (!(pq > 0.f) || !isfinite(pq)) {
@@ -737,11 +746,9 @@ __global__ void __launch_bounds__(32 * kClMaxWarps, 1) ir_cluster_kernel(const C
 #pragma unroll
         for (int i = 0; i < UPW; ++i) {
           if (i < nu) {
-            float pv[NP];
-            cl_load<NP>(P, pplane, slot0 + 32 * i, pv);
 #pragma unroll
             for (int q = 0; q < NP; ++q) {
-              X[i][q] = fmaf(al[q], pv[q], X[i][q]);
+              X[i][q] = fmaf(al[q], D[i][q], X[i][q]);
               R[i][q] = fmaf(-al[q], Q[i][q], R[i][q]);
             }
           }
@@ -991,8 +998,8 @@ __global__ void cl_fill_kernel(int nunit, const int32_t* __restrict__ unit_row, 
 // ---- kernel variants -------------------------------------------------------------
 using ClKernel = void (*)(const ClArgs, int);
 
-// Units a warp holds, by columns: three NP-wide register rows per unit (r, x,
-// and z or q), 36 registers at most, so that 16 warps fit without spilling.
+// Units a warp holds, by columns: four NP-wide register rows per unit (r, x, p,
+// and z or q), 48 registers at most, so that 16 warps fit without spilling.
 struct ClVariant {
   int np, upw;
   ClKernel tl, jacobi;
