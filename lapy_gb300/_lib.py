@@ -199,8 +199,18 @@ def launch_count() -> int:
     return int(lib().lapy_launch_count())
 
 
+_profile_on = False
+
+
 def profile_enable(on: bool = True) -> None:
+    global _profile_on
     lib().lapy_profile_enable(1 if on else 0)
+    _profile_on = bool(on)
+
+
+def profile_enabled() -> bool:
+    """The last state set by ``profile_enable`` in this process."""
+    return _profile_on
 
 
 def profile_reset() -> None:

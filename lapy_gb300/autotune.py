@@ -7,7 +7,8 @@ the device and on the shape of the batch (how many meshes, how large):
 * ``block``        Lanczos block width (columns per inner solve): 2, 4 or 8;
 * ``agg_target``   rows per aggregate of the two-level coarse space;
 * ``round_rtol``   residual reduction of each FP32 refinement round;
-* ``ctas_per_sm``  resident CTAs per SM of the persistent PCG.
+* ``ctas_per_sm``  resident CTAs per SM of the grid-wide PCG (a batch whose
+  meshes all fit on chip does not run it, and this knob is left out).
 
 ``calibrate`` times the solver on a stratified sample of the batch (whole
 meshes, the largest sizes included) by coordinate descent from the defaults,
@@ -33,6 +34,8 @@ import time
 from pathlib import Path
 
 import numpy as np
+
+from . import _lib
 
 DEFAULT = {"block": 4, "agg_target": 64, "round_rtol": 1e-3, "ctas_per_sm": 5}
 CANDIDATES = {
@@ -146,6 +149,20 @@ def timed_trial(fem, k: int, choice: dict, repeats: int = 1, sync=lambda: None) 
     return float(np.median(times))
 
 
+def _grid_wide(fem, k: int) -> bool:
+    """One solve with the default knobs, and whether the grid-wide PCG ran in it
+    (the profile's phase times are that kernel's)."""
+    was = _lib.profile_enabled()
+    before = _lib.profile_read()
+    _lib.profile_enable(True)
+    try:
+        fem.eigs(k=k, block=DEFAULT["block"], tuning=solver_tuning(DEFAULT))
+    finally:
+        _lib.profile_enable(was)
+    after = _lib.profile_read()
+    return any(after[key] > before[key] for key in after if key.startswith("phase_"))
+
+
 def calibrate(meshes, k: int = 50, sample: int = 32, candidates: dict | None = None, cache: TuneCache | None = None,
               repeats: int = 1) -> tuple[dict, list]:
     """Time the candidates on a stratified sample of `meshes` and store the
@@ -157,8 +174,9 @@ def calibrate(meshes, k: int = 50, sample: int = 32, candidates: dict | None = N
     seg = np.cumsum([0] + [len(m.v) for m in meshes])
     idx = stratified_sample(seg, sample)
     fem = BatchedFEM.from_input(BatchInput([meshes[i] for i in idx]), lump=False)
-    fem.eigs(k=k, block=DEFAULT["block"], tuning=solver_tuning(DEFAULT))  # warm-up
-
+    grid_wide = _grid_wide(fem, k)  # also the warm-up
+    if candidates is None:
+        candidates = {key: v for key, v in CANDIDATES.items() if key != "ctas_per_sm" or grid_wide}
     choice, report = descend(lambda c: timed_trial(fem, k, c, repeats, torch.cuda.synchronize),
                              candidates=candidates)
     cache = cache or TuneCache()
