@@ -301,8 +301,6 @@ def run_gpu(args, rank, world):
     if world > 1:
         torch.distributed.barrier()
     L0 = _lib.launch_count()
-    _lib.profile_reset()
-    _lib.profile_enable(True)
     with ClockSampler(torch.cuda.current_device()) as clk:
         torch.cuda.synchronize()
         t0 = time.perf_counter()
@@ -316,10 +314,19 @@ def run_gpu(args, rank, world):
         ev1.record()
         torch.cuda.synchronize()
         wall = time.perf_counter() - t0
-    _lib.profile_enable(False)
-    prof = _lib.profile_read()
     launches = _lib.launch_count() - L0
     dev_s = ev0.elapsed_time(ev1) / 1e3
+    # the solver's counters and timers, from one more step: its timers add a wait per block step
+    _lib.profile_reset()
+    _lib.profile_enable(True)
+    torch.cuda.synchronize()
+    tp = time.perf_counter()
+    step()
+    torch.cuda.synchronize()
+    tp = time.perf_counter() - tp
+    _lib.profile_enable(False)
+    prof = _lib.profile_read()
+    on_chip = not any(v for key, v in prof.items() if key.startswith("phase_"))
     t_max = max_over_ranks(dev_s, world)
     status_ok = all(int(s) == 0 for inf in infos for s in inf["status"])
 
@@ -348,17 +355,19 @@ def run_gpu(args, rank, world):
                    "parallelism": f"replicas x{world} (meshes sharded, no collective)"},
         "e2e": ({"value": world * args.meshes * e2e_steps / te, "unit": "spectra/s", "h2d_bytes_per_step": h2d,
                  "d2h_bytes_per_step": d2h, "calls": e2e_steps} if e2e_steps else None),
-        "roofline": {"bound": "hbm", "kernel": "ir_cluster_kernel (on-chip FP32 two-level PCG)",
-                     "achieved": achieved, "peak": hbm, "unit": "GB/s",
-                     "frac": (achieved / hbm) if achieved else None,
-                     # the algorithm's bytes per second: the solve keeps its matrix and vectors in shared
-                     # memory, so this is no DRAM traffic (none measured) and may pass the copy bandwidth
-                     "traffic": None,
-                     "traffic_unit": "bytes per launch",
+        # on chip the matrix and the vectors are in shared memory and registers: no share of a memory
+        # bandwidth bounds the kernel, its barriers and instruction issue do
+        "roofline": {"bound": "cluster barriers and instruction issue" if on_chip else "hbm",
+                     "kernel": ("ir_cluster_kernel (on-chip FP32 two-level PCG)" if on_chip
+                                else "pcg_kernel (FP32 two-level PCG)"),
+                     "achieved": None if on_chip else achieved, "peak": None if on_chip else hbm, "unit": "GB/s",
+                     "frac": achieved / hbm if achieved and not on_chip else None,
+                     "traffic": None, "traffic_unit": "bytes per launch",
                      "algorithmic_per_launch": (prof["algorithmic_bytes"] / prof["pcg_launches"]
-                                                if prof["pcg_launches"] else None),
+                                                if prof["pcg_launches"] and not on_chip else None),
                      "peak_kind": f"{peak_kind} hbm_gbs",
-                     "pcg_share_of_step": prof["pcg_ms"] / 1e3 / dev_s if dev_s > 0 else None},
+                     "us_per_iteration": 1e3 * prof["pcg_ms"] / prof["pcg_iterations"] if prof["pcg_iterations"] else None,
+                     "pcg_share_of_step": prof["pcg_ms"] / 1e3 / tp if tp > 0 else None},
         "gpu_launches": int(launches),
         "clocks": clk.summary(),
         "status_ok": status_ok,
