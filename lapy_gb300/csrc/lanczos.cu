@@ -1130,7 +1130,8 @@ struct EigOps {
 // m x m projected matrices (1.0 ms at m = 128, 2.1 ms at 224 for one mesh, 3.1
 // ms at 160 for 128 meshes); a block step's fixed cost plus its inner
 // iterations, on chip (0.8 ms at 10,242 rows and 110 iterations, 2.3 ms at
-// 244,228, 10 ms at 1,251,846) or as grid-wide launches.
+// 244,228, 10 ms at 1,251,846, before 5 to 15 % went to plain CG) or as
+// grid-wide launches.
 constexpr double kCheckSecPerDim = 1.0e-5;
 constexpr double kCheckMeshes = 64.0;  // meshes that double a check's time
 constexpr double kChipStepSec = 3.5e-4, kChipIterSec = 4.0e-6, kChipIterSecPerRow = 6.0e-11;
@@ -1622,10 +1623,10 @@ extern "C" int lapy_eigs_shift_invert_tuned(int64_t n, const int32_t* indptr, co
   EigPtrs e;
   layout_eig(P, (char*)(((uintptr_t)ws + 255) & ~uintptr_t(255)), &e);
   EigResult r;
-  // FP32 refinement rounds of 1e-3 (measured on the batched workload: 1e-3 /
-  // 1e-4 / 1e-5 / 2e-3 / 1e-2 per round gave 107 / 101 / 95 / 101 / 99 spectra/s;
-  // tighter rounds spend iterations where FP32 CG stalls, looser ones restart
-  // more often)
+  // FP32 refinement rounds of 1e-3 (on chip, 128 meshes of 642 to 40,962
+  // vertices: 1e-2 / 3e-3 / 2e-3 / 1e-3 / 3e-4 / 1e-4 / 1e-5 per round took 597 /
+  // 579 / 580 / 547 / 563 / 563 / 572 ms; tighter rounds spend iterations where
+  // FP32 CG stalls, looser ones restart more often)
   const double round_rtol = tn.round_rtol > 0.0 ? tn.round_rtol : 1e-3;
   LAPY_TRY(eigs_run(P, e, indptr, indices, a_vals, m_vals, m_is_diag, sigma, tol, inner_rtol, round_rtol,
                     inner_maxiter, seed, evals, evecs, (cudaStream_t)stream, &r));

@@ -24,13 +24,14 @@
 // runs in the same kernel: a solve is one launch per cluster size.
 //
 // Measured per PCG iteration (persistent PCG -> here): one 642-vertex surface,
-// 8 columns, two-level 35 -> 2.5 us; 10,242 vertices 45 -> 4.5 us; 11,466-vertex
-// solid 47 -> 6.0 us; 40,962 vertices, one column, Jacobi 17 -> 3.3 us; 24
-// meshes of 642 to 40,962 vertices, 4 columns 60 -> 14.6 us, 128 of them 106 ->
-// 64 us.  What bounds it now: for small meshes the chain of reductions and
-// barriers (about 500 to 1,000 cycles for each of the three cluster barriers
-// with its reduction); for full CTAs instruction issue and shared-memory
-// wavefronts (both about 40 % busy) between those barriers.
+// 8 columns, two-level 35 -> 2.8 us; 10,242 vertices 45 -> 5.0 us; 11,466-vertex
+// solid 47 -> 6.0 us; 40,962 vertices, one column, Jacobi 17 -> 3.9 us; 24
+// meshes of 642 to 40,962 vertices, 4 columns 60 -> 15 us, 128 of them 106 ->
+// 66 us.  What bounds it now: for small meshes the chain of reductions and
+// barriers; for full CTAs (counters of eight meshes, clusters of 16 CTAs)
+// instruction issue and shared-memory wavefronts, 44 and 35 % of the active
+// cycles, between those barriers: waits for shared memory are first among the
+// stalls, for the CTA's and the cluster's barriers next.
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -348,7 +349,20 @@ __global__ void __launch_bounds__(32 * kClMaxWarps, 1) ir_cluster_kernel(const C
   }
   __syncthreads();
 
-  float R[UPW][NP], X[UPW][NP], D[UPW][NP], dv[UPW], dg[UPW];  // residual, solution, direction
+  // residual, solution, and the direction where its registers are few (geodesics
+  // of 40,962 vertices 9.2 -> 8.5 ms; with 12 a lane the matrix product has fewer
+  // loads in flight: 128 spectra 531 -> 557 ms)
+  constexpr bool kDirRegs = UPW * NP <= 8;
+  float R[UPW][NP], X[UPW][NP], D[kDirRegs ? UPW : 1][NP], dv[UPW], dg[UPW];
+  // the direction in unit i of this warp
+  auto direction = [&](int i, float (&x)[NP]) {
+    if constexpr (kDirRegs) {
+#pragma unroll
+      for (int q = 0; q < NP; ++q) x[q] = D[i][q];
+    } else {
+      cl_load<NP>(P, pplane, slot0 + 32 * i, x);
+    }
+  };
   // global row of unit i of this warp and lane, or -1 past the unit's last row
   auto row_of = [&](int i) -> int64_t {
     if (i >= nu) return -1;
@@ -488,9 +502,16 @@ __global__ void __launch_bounds__(32 * kClMaxWarps, 1) ir_cluster_kernel(const C
     const float rtol2 = (float)(round_rtol * round_rtol);
     // ---- FP32 PCG from zero on R
 #pragma unroll
-    for (int i = 0; i < UPW; ++i)
+    for (int i = 0; i < UPW; ++i) {
+      float zero[NP];
 #pragma unroll
-      for (int q = 0; q < NP; ++q) { X[i][q] = 0.f; D[i][q] = 0.f; }
+      for (int q = 0; q < NP; ++q) {
+        X[i][q] = 0.f;
+        zero[q] = 0.f;
+        if constexpr (kDirRegs) D[i][q] = 0.f;
+      }
+      if (!kDirRegs && i < nu) cl_save<NP>(P, pplane, slot0 + 32 * i, zero);
+    }
     for (int h = threadIdx.x; h < c.nhalo; h += blockDim.x) {
       float zero[NP];
 #pragma unroll
@@ -647,9 +668,14 @@ __global__ void __launch_bounds__(32 * kClMaxWarps, 1) ir_cluster_kernel(const C
 #pragma unroll
         for (int i = 0; i < UPW; ++i) {
           if (i < nu) {
+            float pv[NP];
+            direction(i, pv);
 #pragma unroll
-            for (int q = 0; q < NP; ++q) D[i][q] = fmaf(be[q], D[i][q], z[i][q]);
-            cl_save<NP>(P, pplane, slot0 + 32 * i, D[i]);
+            for (int q = 0; q < NP; ++q) {
+              z[i][q] = fmaf(be[q], pv[q], z[i][q]);
+              if constexpr (kDirRegs) D[i][q] = z[i][q];
+            }
+            cl_save<NP>(P, pplane, slot0 + 32 * i, z[i]);
           }
         }
         if (a.z_halo) {
@@ -663,7 +689,7 @@ __global__ void __launch_bounds__(32 * kClMaxWarps, 1) ir_cluster_kernel(const C
           }
           __syncthreads();
         } else {
-          if (cs > 1) push_rows(D, P, pplane, 1);
+          if (cs > 1) push_rows(z, P, pplane, 1);
           cl_sync(cs);
         }
       }
@@ -712,10 +738,12 @@ __global__ void __launch_bounds__(32 * kClMaxWarps, 1) ir_cluster_kernel(const C
                 Q[i][q] = fmaf(va.y, x1[q], Q[i][q]);
               }
             }
+            float pv[NP];
+            direction(i, pv);
 #pragma unroll
             for (int q = 0; q < NP; ++q) {
-              Q[i][q] = fmaf(dg[i], D[i][q], Q[i][q]);
-              red[q] = fmaf(D[i][q], Q[i][q], red[q]);
+              Q[i][q] = fmaf(dg[i], pv[q], Q[i][q]);
+              red[q] = fmaf(pv[q], Q[i][q], red[q]);
             }
           }
         }
@@ -746,9 +774,11 @@ __global__ void __launch_bounds__(32 * kClMaxWarps, 1) ir_cluster_kernel(const C
 #pragma unroll
         for (int i = 0; i < UPW; ++i) {
           if (i < nu) {
+            float pv[NP];
+            direction(i, pv);
 #pragma unroll
             for (int q = 0; q < NP; ++q) {
-              X[i][q] = fmaf(al[q], D[i][q], X[i][q]);
+              X[i][q] = fmaf(al[q], pv[q], X[i][q]);
               R[i][q] = fmaf(-al[q], Q[i][q], R[i][q]);
             }
           }
@@ -998,8 +1028,9 @@ __global__ void cl_fill_kernel(int nunit, const int32_t* __restrict__ unit_row, 
 // ---- kernel variants -------------------------------------------------------------
 using ClKernel = void (*)(const ClArgs, int);
 
-// Units a warp holds, by columns: four NP-wide register rows per unit (r, x, p,
-// and z or q), 48 registers at most, so that 16 warps fit without spilling.
+// Units a warp holds, by columns: four NP-wide register rows per unit (r, x, z or
+// q, and p where they are few), 36 registers at most, so that 16 warps fit
+// without spilling.
 struct ClVariant {
   int np, upw;
   ClKernel tl, jacobi;
@@ -1129,7 +1160,8 @@ int cluster_plan(int64_t n, int64_t nnz, const int32_t* indptr, const int32_t* i
   // barriers and reductions plus its units' products: measured with two-level
   // clusters of 1 / 8 / 4 CTAs at 21 / 43 / 86 units of 7 entries a row, one
   // column: 2.4 / 4.5 / 5.7 us, two columns: 2.7 / 5.2 / 6.8 us, and 14
-  // entries a row, two columns: 7.5 / 12.5 us at 46 / 92 units.  One mesh is
+  // entries a row, two columns: 7.5 / 12.5 us at 46 / 92 units (with q by
+  // recurrence; 5 to 15 % more since, on all of them).  One mesh is
   // therefore spread over more, narrower clusters until the GPU is full, a
   // batch over as few CTAs as hold it.  Clusters do not cross GPCs: those of
   // 16 CTAs fill 112 of the 152 SMs, of 8 120, of 4 144.
