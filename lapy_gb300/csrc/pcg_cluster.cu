@@ -4,21 +4,21 @@
 // or L2 in each iteration and passes three or four grid barriers; on meshes of
 // a few thousand rows it is bound by those barriers and by dependent L2 round
 // trips (25 to 40 us per iteration for one 642- to 10,242-row mesh).  Here a
-// mesh lives on the SMs of one cluster: the residual, the product vectors and
-// (where registers allow) the solution in registers, one row per lane; the
-// search direction and the preconditioned residual in shared memory, where
-// neighbouring rows are read, through distributed shared memory when another
-// CTA of the cluster owns them; the FP32 matrix with 16-bit column codes in
-// shared memory.  Copies of neighbouring rows' directions are updated where
-// they are read (p = z + beta p; their owners store z), so that r'z is reduced
-// by the barrier that publishes z and q = K p, p'q are computed as plain CG
-// has them: three cluster barriers per iteration with the two-level
-// preconditioner, two with Jacobi (one more where the copies are many).  (The Chronopoulos-Gear form, q by recurrence
-// and p'q = z'K z - beta r'z / alpha_old, needs no more barriers either, but the
-// difference cancels where K is close to singular in FP32: spheres of radius
-// 0.02 and 0.03 at sigma = -0.01 took up to 25 times the iterations or failed.)
-// Every CTA adds the partial sums of all CTAs in rank order, so each takes the
-// same decisions and a solve is reproducible to the bit.
+// mesh lives on the SMs of one cluster: the residual, the solution and (where
+// registers allow) the search direction in registers, one row per lane; the
+// direction in shared memory too, where neighbouring rows are read; copies of the
+// rows that other CTAs of the cluster own; the FP32 matrix with 16-bit column
+// codes in shared memory.  Copies of directions are updated where they are read
+// (p = z + beta p; their owners store z through distributed shared memory), so
+// that r'z is reduced by the barrier that publishes z, and q = K p, p'q are
+// computed as plain CG has them: three cluster barriers per iteration with the
+// two-level preconditioner, two with Jacobi (one more where the copies are
+// many).  (The Chronopoulos-Gear form, q by recurrence and p'q = z'K z - beta r'z
+// / alpha_old, needs no more barriers either, but the difference cancels where K
+// is close to singular in FP32: spheres of radius 0.02 and 0.03 at sigma = -0.01
+// took up to 25 times the iterations or failed.)  Every CTA adds the partial sums
+// of all CTAs in one order, so each takes the same decisions and a solve is
+// reproducible to the bit.
 //
 // The FP64 refinement (true residual B - K X in FP64, FP32 correction solves)
 // runs in the same kernel: a solve is one launch per cluster size.
@@ -26,10 +26,10 @@
 // Measured per PCG iteration (persistent PCG -> here): one 642-vertex surface,
 // 8 columns, two-level 35 -> 2.8 us; 10,242 vertices 45 -> 5.0 us; 11,466-vertex
 // solid 47 -> 6.0 us; 40,962 vertices, one column, Jacobi 17 -> 3.9 us; 24
-// meshes of 642 to 40,962 vertices, 4 columns 60 -> 15 us, 128 of them 106 ->
-// 66 us.  What bounds it now: for small meshes the chain of reductions and
+// meshes of 642 to 40,962 vertices, 4 columns 60 -> 14 us, 128 of them 106 ->
+// 62 us.  What bounds it now: for small meshes the chain of reductions and
 // barriers; for full CTAs (counters of eight meshes, clusters of 16 CTAs)
-// instruction issue and shared-memory wavefronts, 44 and 35 % of the active
+// instruction issue and shared-memory wavefronts, 42 % each of the active
 // cycles, between those barriers: waits for shared memory are first among the
 // stalls, for the CTA's and the cluster's barriers next.
 #include <algorithm>
